@@ -13,20 +13,30 @@
 // quadrature grid.  BP2/BP4 apply the same operator to each of the 3 fields.
 //
 // Work mapping.  Every 1D step (interpolation, derivative, projection, weak
-// derivative) is a small matrix applied along lines of the element's grid.
-// A thread owns whole lines: it reads one line into registers and writes all
-// of that line's outputs, so the matrix index of every multiply-add is the
-// same in all threads of the warp.  The matrices therefore live in the
-// constant bank (c_cub below), read uniformly through the constant cache;
-// shared memory only carries the field between steps whose line direction
-// changes.
-// The G x G threads of an element slot take the roles
-//   (b-line of node a, c) -> (a-line of point j, c) -> (c-line of point i, j)
-// through the interpolation, keep the c-line (the t-direction) in registers
-// for the t-derivative and the t-part of the weak divergence, and run the
-// r- and s-parts as row/column roles over shared memory.  The projection runs
-// the same roles backwards and ends on b-lines of node (a, c), the lines the
-// thread loaded q along; its q.Aq sum for the fused CG re-reads q there.
+// derivative) is a small matrix applied along lines of the element's grid.  A
+// thread owns one line of every step: it reads the line into registers and
+// writes all of its outputs, so the matrix index of every multiply-add is the
+// same in all threads of the warp and the matrices live in the constant bank
+// (c_cub below); shared memory only carries the field between steps whose line
+// direction changes.  The steps of one (element, field):
+//   b-lines of nodes (a, c), a-lines (j, c), c-lines (i, j)   interpolation
+//   rows (y, z), columns (x, z)                                r-, s-derivative
+//   columns (x, y)     t-derivative, fluxes, t-part of the weak divergence
+//   rows, columns                                              r-, s-part added
+//   columns (x, z), (x, b), rows (b, c)                        projection
+// The mass forms go from the c-line to the points and back in registers.
+//
+// What bounds it: the FP64 stiffness at p=7 moves 50 KB of factors and values
+// and 25 passes of 8 bytes per point through shared memory; DRAM, the shared-
+// memory pipe and FP64 arithmetic need 0.49, 0.3 and 0.3 ms of a 40^3 launch.
+// What it takes is many independent warps with few registers: one element per
+// block of three warps keeps 18-24 warps per SM resident, and a bulk prefetch
+// asks L2 for the element's factors while q is gathered and interpolated, so
+// the flux loop reads them without a trip to DRAM.  Measured at 40^3 curved
+// p=7 (before: three elements in lockstep per block of 243 threads, outer
+// loops rolled for registers, 16 warps): BK3 FP64 1.376 -> 0.79 ms, BK1 at
+// 32^3 365 -> 131 us, FP32 BK3 at 19x19x20 87 -> 61 us; BK4 p=5 on 21x18x23
+// 221 -> 147 us.
 #pragma once
 
 #ifndef BP_CUB_REAL
@@ -45,16 +55,6 @@ namespace bp {
 namespace {
 
 using CubReal = BP_CUB_REAL;
-
-// Outer (output) loops of the line steps.  Fully unrolled, every matrix index
-// is a compile-time constant, but the unrolled FP64 steps need more registers
-// than two resident blocks allow; measured at p=7 (BK3 40^3 curved): FP64
-// 1.4 ms rolled against 2.1-2.2 ms unrolled, FP32 (mixed BP3 CG to 1e-8)
-// 1.57 s unrolled against 1.81 s rolled.  So FP64 keeps them rolled and FP32
-// unrolls them.
-#ifndef BP_CUB_OUTER
-#define BP_CUB_OUTER _Pragma("unroll 1")
-#endif
 
 enum CubForm { CUB_MASS_AFFINE = 0, CUB_MASS = 1, CUB_STIFF_AFFINE = 2, CUB_STIFF = 3 };
 
@@ -86,309 +86,88 @@ static_assert(kCubTable * sizeof(double) <= 64 * 1024, "constant table exceeds t
 
 static __constant__ CubReal c_cub[kCubTable];
 
+// Slots per block, registers a thread may take and unrolling, by the points G
+// per direction (sweeps over all degrees, 10^3..60^3 boxes, both precisions;
+// GB/s of the byte model).  Several slots only where one leaves the block
+// small (a mass element of 9 threads: 28 slots 2940 GB/s, 7 slots 1950; the
+// counts divide by three there, so that the fields of an element share a
+// block's L1) or a
+// warp half empty (G = 6: 36 threads).  Registers: the least that does not
+// spill, for more resident blocks (FP64 stiffness G = 9: 96 registers 4002,
+// 80 3726 GB/s; G = 10: 96 3855, 128 3620).  Outputs of a line are unrolled but
+// for FP64 G = 13 and 17 and FP32 G = 12..14 (spills: FP32 G = 13 1979 against
+// 2024 GB/s rolled by three); the flux loop runs three points at a time, the
+// mass columns as a whole (FP64 G = 11: 3083 against 2946 GB/s by three),
+// except where that spills (G = 16: 350 against 62 us).
+template <int NQ, int FORM>
+struct CubRule {
+  static constexpr bool CURVED = (FORM == CUB_MASS || FORM == CUB_STIFF);
+  static constexpr bool STIFF = (FORM == CUB_STIFF_AFFINE || FORM == CUB_STIFF);
+  static constexpr bool D = sizeof(CubReal) == 8;
+  static constexpr int G = CURVED ? NQ + 1 : NQ;
+  static constexpr int EPB = STIFF ? (G == 2 ? 24 : G == 3 ? 21 : G == 4 ? 6 : G <= 6 ? 5 : G == 8 && D ? 2 : 1)
+                                   : (G == 2 ? 24 : G == 3 ? 21 : G == 4 ? 12 : G <= 6 ? 5 : G == 7 ? 3 : G == 8 ? 2 : 1);
+  static constexpr int WARPS = (G * G * EPB + 31) / 32;
+  static constexpr int REGS = !D ? (G <= 7 ? 48 : 3 * G + 26) : !STIFF ? 4 * G + 24 : G <= 6 ? 64 : G == 7 ? 80 : G <= 13 ? 100 : G <= 16 ? 128 : 170;
+  static constexpr int minb(bool dot) {   // resident blocks to allow for (the q.Aq form takes 8 registers more)
+    const int n = 65536 / (WARPS * 32 * (REGS + (dot ? 8 : 0)));
+    return n < 1 ? 1 : n * WARPS > 64 ? 64 / WARPS : n > 32 ? 32 : n;
+  }
+  static constexpr int UN = STIFF && (D ? G == 13 || G == 17 : G >= 12 && G <= 14) ? 3 : G;
+  static constexpr int UK = STIFF ? (G == 6 ? 1 : 3) : G == 16 ? 3 : G;
+};
+
+// One element (of one field) per slot of G x G threads, EPB slots per block.
 template <int NQ, int FORM>
 struct CubShape {
   static constexpr bool CURVED = (FORM == CUB_MASS || FORM == CUB_STIFF);
   static constexpr bool STIFF = (FORM == CUB_STIFF_AFFINE || FORM == CUB_STIFF);
   static constexpr int G = CURVED ? NQ + 1 : NQ;   // quadrature points per direction
-  static constexpr int G2 = G * G;
-  static constexpr int RS = (G % 2) ? G : G + 1;   // row stride: odd, so rows of a warp spread over banks
-  static constexpr int PLANE = G * RS;
-  static constexpr int FIELD = G * PLANE;           // one G^3 field in shared memory
-  static constexpr int NBUF = STIFF ? 3 : 1;        // u, and the r/s buffers of the stiffness
-  // words between consecutive element slots' buffers beyond NBUF fields: the
-  // warps that straddle two slots then spread their shared-memory accesses
-  // over more banks (padding chosen per Nq by counting the wavefronts of every
-  // access pattern of the FP32 kernels: 12-25% fewer at Nq = 2, 4, 5, 6, 8)
-  static constexpr int SPAD = sizeof(CubReal) != 4 ? 0
-                              : NQ == 2 ? 10 : NQ == 4 ? 2 : NQ == 5 ? 8 : NQ == 6 ? 12 : NQ == 8 ? 6 : NQ == 9 ? 8 : 0;
-  static constexpr int SLOTW = NBUF * FIELD + SPAD;   // words per element slot
-  static constexpr int EPB0 = 256 / G2 < 1 ? 1 : 256 / G2;
-  static constexpr int EPB = EPB0 > 8 ? 8 : EPB0;   // element slots per block
-  static constexpr int THREADS = G2 * EPB;
-  // resident blocks per SM the register budget must allow (caps registers per thread)
-  static constexpr int MINB = G <= 12 ? 2 : 1;
+  static constexpr int G2 = G * G, GP = G * G2, NP = NQ * NQ * NQ;
+  // row and plane strides of a G^3 field: the rows, columns and lines that a
+  // warp's threads walk fall in distinct banks where that is possible (strides
+  // chosen by counting the wavefronts of every access of the kernel for all
+  // row strides G..G+2 and plane pads 0..15; at even G a stride of G + 1 or a
+  // pad cuts them by 5-20%)
+  static constexpr int RS = (G % 2 || G == 6 || G == 10 || G == 14) ? G : G + 1;
+  static constexpr int PAD = G == 6 ? 1 : G == 7 ? 5 : G == 10 ? 5 : G == 14 ? 9 : G == 16 ? 15 : 0;
+  static constexpr int PL = G * RS + PAD;
+  static constexpr int FIELD = G * PL;
+  static constexpr int NBUF = STIFF ? 3 : 1;        // u, and the r and s buffers of the stiffness
+  static constexpr int EPB = CubRule<NQ, FORM>::EPB;
+  static constexpr int THREADS = (G2 * EPB + 31) / 32 * 32;   // whole warps; the last threads own no line
+  static constexpr size_t FIELDS = sizeof(CubReal) * (size_t)NBUF * FIELD * EPB;
+  static constexpr size_t SMEM = FIELDS < sizeof(double) * THREADS ? sizeof(double) * THREADS : FIELDS;
   static constexpr int SLOT = cub_slot(NQ, FORM);
   static constexpr int TSIZE = G * NQ;              // T rows = output points
   static constexpr int DSIZE = STIFF ? G * G : 0;
-  // FP32 curved forms stage each element's Gauss-point factors in shared memory
-  // with cp.async at the element's start, so their latency overlaps the gather
-  // and the interpolation (the FP64 factors would halve the resident blocks)
-  static constexpr bool STAGE = CURVED && sizeof(CubReal) == 4;
-  static constexpr int GP = G * G * G;
-  static constexpr size_t FIELDS = sizeof(CubReal) * (size_t)SLOTW * EPB;
-  static constexpr size_t GOFF = (FIELDS + 15) & ~(size_t)15;                        // [EPB][GP*6] ggeo
-  static constexpr size_t WOFF = GOFF + (STAGE && STIFF ? sizeof(CubReal) * (size_t)EPB * GP * 6 : 0);   // [EPB][GP] wJ
-  static constexpr size_t SMEM = STAGE ? WOFF + sizeof(CubReal) * (size_t)EPB * GP : FIELDS;
-  // The pipelined FP32 form (ax_cub_pipe_kernel): the element groups' indices
-  // and gathered q, double-buffered, and a ring of element ids behind the
-  // staged factors.
-  static constexpr int NP = NQ * NQ * NQ;
-  static constexpr size_t IOFF = (SMEM + 15) & ~(size_t)15;                 // [EPB][NP] GlobalToLocal
-  static constexpr size_t QOFF = IOFF + sizeof(int32_t) * (size_t)EPB * NP;   // [2][EPB][NP] q
-  static constexpr size_t EOFF = QOFF + sizeof(CubReal) * 2 * (size_t)EPB * NP;   // [4][EPB] element ids
-  static constexpr size_t PSMEM = EOFF + sizeof(int32_t) * 4 * (size_t)EPB;
-  // blocks per SM that shared memory allows (228 KB per SM, 1 KB reserved per
-  // block); the pipelined form is used only where it keeps the slot kernel's
-  // residency (Nq = 10 would fall from two blocks to one, Nq = 16 not fit)
-  static constexpr int smem_blocks(size_t bytes) { return (int)((228 * 1024) / (bytes + 1024)); }
-  static constexpr int min_(int a, int b) { return a < b ? a : b; }
-  static constexpr bool PIPE_OK =
-      PSMEM <= 227 * 1024 && min_(smem_blocks(PSMEM), MINB) >= min_(smem_blocks(SMEM), MINB);
 };
-
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 // The 1D matrices of a form in the constant bank: T(o, i) maps NQ nodes to G
-// points (MASS_AFFINE applies MM^T), D(a, b) is G x G; AT indexes a G^3 field.
-#define CUB_T(o, i)                                                          \
-  (FORM == CUB_MASS_AFFINE ? c_cub[CubShape<NQ, FORM>::SLOT + (i) * NQ + (o)] \
-                           : c_cub[CubShape<NQ, FORM>::SLOT + (o) * NQ + (i)])
-#define CUB_D(a, b) c_cub[CubShape<NQ, FORM>::SLOT + CubShape<NQ, FORM>::TSIZE + (a) * CubShape<NQ, FORM>::G + (b)]
-#define CUB_AT(B, z, y, x) B[(z) * CubShape<NQ, FORM>::PLANE + (y) * CubShape<NQ, FORM>::RS + (x)]
+// points (MASS_AFFINE applies MM^T), D(a, b) is G x G.
+#define CUB_T(o, i) \
+  (FORM == CUB_MASS_AFFINE ? c_cub[Sh::SLOT + (i) * NQ + (o)] : c_cub[Sh::SLOT + (o) * NQ + (i)])
+#define CUB_D(a, b) c_cub[Sh::SLOT + Sh::TSIZE + (a) * Sh::G + (b)]
 
-// Interpolation of one element slot to its G^3 points: along b from the
-// q-line qb of node (a, c) = (tx, ty) (threads tx, ty < NQ), along a over
-// shared memory (rows (j, c) = (tx, ty)), along c into the register column qk
-// of point (i, j) = (tx, ty).  Reads of U after the call are the thread's own
-// column.
-template <int NQ, int FORM>
-__device__ __forceinline__ void cub_interp(const CubReal (&qb)[NQ], CubReal* U,
-                                           CubReal (&qk)[CubShape<NQ, FORM>::G], int tx, int ty) {
-  using F = CubReal;
-  constexpr int G = CubShape<NQ, FORM>::G;
-  if (tx < NQ && ty < NQ) {
-BP_CUB_OUTER
-    for (int jj = 0; jj < G; ++jj) {
-      F t = 0;
+// A line of NI values through the NO x NI matrix mat(o, n): store(o, value).
+template <int NI, int NO, int UN, class F, class Mat, class Store>
+__device__ __forceinline__ void cub_line(const F (&r)[NI], Mat mat, Store store) {
+#pragma unroll UN
+  for (int o = 0; o < NO; ++o) {
+    F a = 0;
 #pragma unroll
-      for (int b = 0; b < NQ; ++b) t += CUB_T(jj, b) * qb[b];
-      CUB_AT(U, ty, jj, tx) = t;
-    }
-  }
-  __syncthreads();
-  if (ty < NQ) {
-    F r[NQ];
-#pragma unroll
-    for (int a = 0; a < NQ; ++a) r[a] = CUB_AT(U, ty, tx, a);
-BP_CUB_OUTER
-    for (int ii = 0; ii < G; ++ii) {
-      F t = 0;
-#pragma unroll
-      for (int a = 0; a < NQ; ++a) t += CUB_T(ii, a) * r[a];
-      CUB_AT(U, ty, tx, ii) = t;
-    }
-  }
-  __syncthreads();
-  F r[NQ];
-#pragma unroll
-  for (int c = 0; c < NQ; ++c) r[c] = CUB_AT(U, c, ty, tx);
-#pragma unroll
-  for (int k = 0; k < G; ++k) {
-    F t = 0;
-#pragma unroll
-    for (int c = 0; c < NQ; ++c) t += CUB_T(k, c) * r[c];
-    qk[k] = t;
+    for (int n = 0; n < NI; ++n) a += mat(o, n) * r[n];
+    store(o, a);
   }
 }
-
-// Factors at the points of column (tx, ty), three sources.  ready() runs before
-// the barrier ahead of the flux loop, released() after the barrier behind it
-// (no thread reads factors after that).
-template <class F>
-struct CubStagedFactors {   // staged in shared memory by cp.async at the element's start
-  const F* sG;
-  const F* sW;
-  __device__ __forceinline__ void ready() const { cp_async_wait_all(); }
-  __device__ __forceinline__ void released() const {}
-  __device__ __forceinline__ void get(int pt, F (&g)[6], F& w) const {
-    using V2 = typename std::conditional<sizeof(F) == 8, double2, float2>::type;
-    const V2* gv = reinterpret_cast<const V2*>(sG + 6 * pt);
-    const V2 a0 = gv[0], a1 = gv[1], a2 = gv[2];
-    g[0] = a0.x; g[1] = a0.y; g[2] = a1.x; g[3] = a1.y; g[4] = a2.x; g[5] = a2.y;
-    w = sW[pt];
-  }
-};
-template <class F>
-struct CubGlobalFactors {   // read from global memory at the flux loop
-  const F* ggeo;              // the element's block
-  const F* wJ;
-  __device__ __forceinline__ void ready() const {}
-  __device__ __forceinline__ void released() const {}
-  __device__ __forceinline__ void get(int pt, F (&g)[6], F& w) const {
-    using V2 = typename std::conditional<sizeof(F) == 8, double2, float2>::type;
-    const V2* gv = reinterpret_cast<const V2*>(ggeo + 6 * pt);
-    const V2 a0 = gv[0], a1 = gv[1], a2 = gv[2];
-    g[0] = a0.x; g[1] = a0.y; g[2] = a1.x; g[3] = a1.y; g[4] = a2.x; g[5] = a2.y;
-    w = wJ[pt];
-  }
-};
-template <class F>
-struct CubAffineFactors {   // one set per element, in registers
-  F ga[6];
-  F wa;
-  __device__ __forceinline__ void ready() const {}
-  __device__ __forceinline__ void released() const {}
-  __device__ __forceinline__ void get(int, F (&g)[6], F& w) const {
+template <int N, int STRIDE, class F>
+__device__ __forceinline__ void cub_load(const F* p, F (&r)[N]) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) g[c] = ga[c];
-    w = wa;
-  }
-};
-
-// Stiffness plus lambda mass at the points of column (i, j) = (tx, ty):
-// acc = Dr^T(G00 dr + G01 ds + G02 dt) + Ds^T(...) + Dt^T(...) + lambda w qk.
-// The r- and s-parts run over shared memory (U, R, S), the t-part in
-// registers; U's own column receives qk first.
-template <int NQ, int FORM, class Fac>
-__device__ __forceinline__ void cub_stiff(const CubReal (&qk)[CubShape<NQ, FORM>::G],
-                                          CubReal (&acc)[CubShape<NQ, FORM>::G], CubReal* U, CubReal* R,
-                                          CubReal* S, int tx, int ty, CubReal lambda, const Fac& fac) {
-  using F = CubReal;
-  constexpr int G = CubShape<NQ, FORM>::G;
-  // own column: every earlier read of it was this thread's
-#pragma unroll
-  for (int k = 0; k < G; ++k) CUB_AT(U, k, ty, tx) = qk[k];
-  __syncthreads();
-  // r-derivative on the row (y, z) = (tx, ty); s-derivative on the column (x, z) = (tx, ty)
-  {
-    F r[G];
-#pragma unroll
-    for (int n = 0; n < G; ++n) r[n] = CUB_AT(U, ty, tx, n);
-BP_CUB_OUTER
-    for (int i = 0; i < G; ++i) {
-      F t = 0;
-#pragma unroll
-      for (int n = 0; n < G; ++n) t += CUB_D(i, n) * r[n];
-      CUB_AT(R, ty, tx, i) = t;
-    }
-#pragma unroll
-    for (int n = 0; n < G; ++n) r[n] = CUB_AT(U, ty, n, tx);
-BP_CUB_OUTER
-    for (int j = 0; j < G; ++j) {
-      F t = 0;
-#pragma unroll
-      for (int n = 0; n < G; ++n) t += CUB_D(j, n) * r[n];
-      CUB_AT(S, ty, j, tx) = t;
-    }
-  }
-  // t-derivative on the column (x, y) = (tx, ty) in registers, from U's own
-  // column (which keeps qk until the projection) rather than from registers
-  // held through the r/s phase
-  F gt[G];
-  {
-    F u[G];
-#pragma unroll
-    for (int n = 0; n < G; ++n) u[n] = CUB_AT(U, n, ty, tx);
-#pragma unroll
-    for (int k = 0; k < G; ++k) {
-      F t = 0;
-#pragma unroll
-      for (int n = 0; n < G; ++n) t += CUB_D(k, n) * u[n];
-      gt[k] = t;
-    }
-  }
-  fac.ready();   // this thread's copies; the barrier below makes all visible
-  __syncthreads();
-  // fluxes at the points of column (tx, ty)
-#pragma unroll
-  for (int k = 0; k < G; ++k) {
-    F g[6], w;
-    fac.get(k * G * G + ty * G + tx, g, w);
-    const F dr = CUB_AT(R, k, ty, tx), ds = CUB_AT(S, k, ty, tx), dt = gt[k];
-    CUB_AT(R, k, ty, tx) = g[0] * dr + g[1] * ds + g[2] * dt;
-    CUB_AT(S, k, ty, tx) = g[1] * dr + g[3] * ds + g[4] * dt;
-    gt[k] = g[2] * dr + g[4] * ds + g[5] * dt;
-    acc[k] = lambda * w * CUB_AT(U, k, ty, tx);
-  }
-  // t-part of the weak divergence, in registers
-#pragma unroll
-  for (int n = 0; n < G; ++n) {
-    F t = acc[n];
-#pragma unroll
-    for (int k = 0; k < G; ++k) t += CUB_D(k, n) * gt[k];
-    acc[n] = t;
-  }
-  __syncthreads();
-  fac.released();
-  // r-part on rows, s-part on columns, in place
-  {
-    F r[G];
-#pragma unroll
-    for (int n = 0; n < G; ++n) r[n] = CUB_AT(R, ty, tx, n);
-BP_CUB_OUTER
-    for (int i = 0; i < G; ++i) {
-      F t = 0;
-#pragma unroll
-      for (int n = 0; n < G; ++n) t += CUB_D(n, i) * r[n];
-      CUB_AT(R, ty, tx, i) = t;
-    }
-#pragma unroll
-    for (int n = 0; n < G; ++n) r[n] = CUB_AT(S, ty, n, tx);
-BP_CUB_OUTER
-    for (int j = 0; j < G; ++j) {
-      F t = 0;
-#pragma unroll
-      for (int n = 0; n < G; ++n) t += CUB_D(n, j) * r[n];
-      CUB_AT(S, ty, j, tx) = t;
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < G; ++k) acc[k] += CUB_AT(R, k, ty, tx) + CUB_AT(S, k, ty, tx);
+  for (int n = 0; n < N; ++n) r[n] = p[n * STRIDE];
 }
 
-// Projection to the nodes along c (from the register column acc of point
-// (i, j) = (tx, ty)) and along a (rows (j, c) = (tx, ty)); the caller
-// finishes along b from U: node (a, c) = (tx, ty) reads U(c, :, a).
-template <int NQ, int FORM>
-__device__ __forceinline__ void cub_project_ca(const CubReal (&acc)[CubShape<NQ, FORM>::G], CubReal* U, int tx,
-                                               int ty) {
-  using F = CubReal;
-  constexpr int G = CubShape<NQ, FORM>::G;
-  // own column of U
-BP_CUB_OUTER
-  for (int c = 0; c < NQ; ++c) {
-    F t = 0;
-#pragma unroll
-    for (int k = 0; k < G; ++k) t += CUB_T(k, c) * acc[k];
-    CUB_AT(U, c, ty, tx) = t;
-  }
-  __syncthreads();
-  if (ty < NQ) {
-    F r[G];
-#pragma unroll
-    for (int ii = 0; ii < G; ++ii) r[ii] = CUB_AT(U, ty, tx, ii);
-BP_CUB_OUTER
-    for (int a = 0; a < NQ; ++a) {
-      F t = 0;
-#pragma unroll
-      for (int ii = 0; ii < G; ++ii) t += CUB_T(ii, a) * r[ii];
-      CUB_AT(U, ty, tx, a) = t;
-    }
-  }
-  __syncthreads();
-}
-
-template <int NQ, int FORM>
-__global__ void __launch_bounds__(CubShape<NQ, FORM>::THREADS, CubShape<NQ, FORM>::MINB)
+template <int NQ, int FORM, bool DOT>
+__global__ void __launch_bounds__((CubShape<NQ, FORM>::THREADS), (CubRule<NQ, FORM>::minb(DOT)))
 ax_cub_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
               const CubReal* __restrict__ wJ, const CubReal* __restrict__ ggeo, CubReal lambda,
               const CubReal* __restrict__ q, CubReal* __restrict__ Aq, const int* __restrict__ skip,
@@ -398,303 +177,222 @@ ax_cub_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementLis
   if (skip && *skip) return;
   using F = CubReal;
   using Sh = CubShape<NQ, FORM>;
-  constexpr int G = Sh::G, GP = Sh::GP, EPB = Sh::EPB;
-  constexpr int NQ2 = NQ * NQ, NP = NQ * NQ * NQ;
-
+  using V2 = typename std::conditional<sizeof(F) == 8, double2, float2>::type;
+  constexpr int G = Sh::G, G2 = Sh::G2, GP = Sh::GP, NQ2 = NQ * NQ, NP = Sh::NP, RS = Sh::RS, PL = Sh::PL;
+  constexpr int EPB = Sh::EPB, UN = CubRule<NQ, FORM>::UN, UK = CubRule<NQ, FORM>::UK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  F* const sbase = reinterpret_cast<F*>(smem_raw);
-  const int tx = threadIdx.x, ty = threadIdx.y, es = threadIdx.z;
-  F* const U = sbase + (size_t)es * Sh::SLOTW;   // the field
+  // The guards t < G2 (hi < G, ...) are also what keeps the steps apart: as one
+  // straight line of code the scheduler moved loads and addresses of later
+  // steps up and spilled (BK3 p=7: 854 against 752 us).
+  const int slot = EPB == 1 || threadIdx.x >= G2 * EPB ? 0 : threadIdx.x / G2;
+  const int t = threadIdx.x - slot * G2;      // >= G2: no line
+  F* const U = reinterpret_cast<F*>(smem_raw) + (size_t)slot * Sh::NBUF * Sh::FIELD;   // the field
   F* const R = U + Sh::FIELD;                                // r-derivative / r-flux
   F* const S = R + Sh::FIELD;                                // s-derivative / s-flux
-
-  const int eidx = blockIdx.x * EPB + es;
-  const bool valid = eidx < Nelements;
+  const int64_t v = (int64_t)blockIdx.x * EPB + slot;        // element-major (element, field)
+  const bool valid = v < (int64_t)Nelements * Nfields;
+  const int eidx = Nfields == 1 ? (int)v : (int)(v / Nfields), f = (int)(v - (int64_t)eidx * Nfields);
   const int element = valid ? elementList[eidx] : 0;
+  const size_t lbase = ((size_t)element * Nfields + f) * NP;
+  const F* const ge = ggeo + 6 * (size_t)element * (Sh::CURVED ? GP : 1);
+  const F* const we = wJ + (size_t)element * (Sh::CURVED ? GP : 1);
+  if (Sh::CURVED && valid && t == 0) {   // the element's factors, while q is gathered and interpolated
+    if (Sh::STIFF) l2_prefetch(ge, 6 * GP);
+    l2_prefetch(we, GP);
+  }
+  // line (y, z), (x, z) or (x, y) of this thread in the roles of the steps
+  // G x G lines hi < G; G x NQ lines hi < NQ; NQ x NQ lines hn < NQ
+  const int hi = t / G, lo = t - hi * G, hn = t / NQ, ln = t - hn * NQ;
+  const auto T = [](int o, int i) { return CUB_T(o, i); };
+  const auto Tt = [](int o, int i) { return CUB_T(i, o); };
+  const auto D = [](int o, int i) { return CUB_D(o, i); };
+  const auto Dt = [](int o, int i) { return CUB_D(i, o); };
   double pdot = 0.0;
+  // q.A_e q, where its factors are in registers: at the points, lambda w (I q)^2
+  // and the gradient times the flux (the affine mass has no such place and
+  // gathers q again)
 
-  // the element's factors into shared memory, in flight while q is gathered and interpolated
-  F* const sG = reinterpret_cast<F*>(smem_raw + Sh::GOFF) + (size_t)es * GP * 6;
-  F* const sW = reinterpret_cast<F*>(smem_raw + Sh::WOFF) + (size_t)es * GP;
-  if (Sh::STAGE && valid) {
-    const int tl = tx + G * ty;
-    if (Sh::STIFF) {
-      const F* src = ggeo + 6 * (size_t)element * GP;   // 8-byte aligned: 24 bytes per point
-      for (int c = tl; c < GP * 3; c += G * G) cp_async8(sG + 2 * c, src + 2 * c);
-    }
-    const F* srcw = wJ + (size_t)element * GP;
-    for (int c = tl; c < GP; c += G * G) cp_async4(sW + c, srcw + c);
+  // interpolation: along b from the gathered nodes (a, c) = (ln, hn)
+  if (hn < NQ) {
+    int32_t id[NQ];
+    F r[NQ];
+#pragma unroll
+    for (int b = 0; b < NQ; ++b) id[b] = valid ? __ldg(G2L + lbase + hn * NQ2 + b * NQ + ln) : -1;
+#pragma unroll
+    for (int b = 0; b < NQ; ++b) r[b] = id[b] >= 0 ? __ldg(q + id[b]) : F(0);
+    F* const p = U + hn * PL + ln;
+    cub_line<NQ, G, UN>(r, T, [&](int o, F x) { p[o * RS] = x; });
   }
-
-  for (int f = 0; f < Nfields; ++f) {
-    const size_t lbase = ((size_t)element * Nfields + f) * NP;
-    if (f > 0) __syncthreads();   // the previous field's last reads of U are done
-    // q[c][b][a] along b of node (a, c) = (tx, ty)
-    F qb[NQ];
-#pragma unroll
-    for (int b = 0; b < NQ; ++b) {
-      F v = 0;
-      if (valid && tx < NQ && ty < NQ) {
-        const int32_t id = G2L[lbase + ty * NQ2 + b * NQ + tx];
-        v = (id >= 0) ? q[id] : F(0);
-      }
-      qb[b] = v;
-    }
-    F qk[G];
-    cub_interp<NQ, FORM>(qb, U, qk, tx, ty);
-    if (FORM == CUB_MASS_AFFINE) {
-      // G == NQ: the result column of node (tx, ty) is wJ_e * qk
-      if (valid) {
-        const F wa = wJ[element];
-#pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          const F out = wa * qk[k];
-          const size_t l = lbase + k * NQ2 + ty * NQ + tx;
-          Aq[l] = out;
-          if (partials) {
-            const int32_t id = G2L[l];
-            pdot += (double)(id >= 0 ? q[id] : F(0)) * (double)out;
-          }
-        }
-      }
-      continue;
-    }
-    F acc[G];
-    if (FORM == CUB_MASS) {
-      if (Sh::STAGE) {
-        cp_async_wait_all();
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < G; ++k) acc[k] = sW[k * G * G + ty * G + tx] * qk[k];
-      } else {
-        const size_t gb = (size_t)element * GP + ty * G + tx;
-#pragma unroll
-        for (int k = 0; k < G; ++k) acc[k] = wJ[gb + k * G * G] * qk[k];
-      }
-    } else if (Sh::STAGE) {
-      cub_stiff<NQ, FORM>(qk, acc, U, R, S, tx, ty, lambda, CubStagedFactors<F>{sG, sW});
-    } else if (Sh::CURVED) {
-      cub_stiff<NQ, FORM>(qk, acc, U, R, S, tx, ty, lambda,
-                          CubGlobalFactors<F>{ggeo + 6 * (size_t)element * GP, wJ + (size_t)element * GP});
-    } else {
-      CubAffineFactors<F> fa;
-#pragma unroll
-      for (int c = 0; c < 6; ++c) fa.ga[c] = ggeo[6 * (size_t)element + c];
-      fa.wa = wJ[element];
-      cub_stiff<NQ, FORM>(qk, acc, U, R, S, tx, ty, lambda, fa);
-    }
-    cub_project_ca<NQ, FORM>(acc, U, tx, ty);
-    // along b: node (a, c) = (tx, ty), the line q was loaded along
-    if (tx < NQ && ty < NQ && valid) {
-      F r[G];
-#pragma unroll
-      for (int jj = 0; jj < G; ++jj) r[jj] = CUB_AT(U, ty, jj, tx);
-#pragma unroll
-      for (int b = 0; b < NQ; ++b) {
-        F t = 0;
-#pragma unroll
-        for (int jj = 0; jj < G; ++jj) t += CUB_T(jj, b) * r[jj];
-        const size_t l = lbase + ty * NQ2 + b * NQ + tx;
-        Aq[l] = t;
-        if (partials) {   // q again (a cache hit) rather than a line held in registers throughout
-          const int32_t id = G2L[l];
-          pdot += (double)(id >= 0 ? q[id] : F(0)) * (double)t;
-        }
-      }
-    }
-  }
-  if (partials) {
-    static_assert(Sh::FIELDS >= sizeof(double) * Sh::THREADS, "scratch too small");
-    const double bs = fuse_block_sum(pdot, reinterpret_cast<double*>(sbase));
-    if (tx == 0 && ty == 0 && es == 0) partials[blockIdx.x] = bs;
-  }
-}
-
-// Curved stiffness (BP3, one field, even Nq) with the memory traffic of the
-// next element groups in flight while a group computes.  A resident grid of
-// blocks loops over groups of EPB elements; with iteration i of a block on
-// group h_i = blockIdx.x + i gridDim.x, the pipeline holds
-//   element ids of h_{i+3}  -> sEl[(i+3) & 3]   (4-byte copies)
-//   GlobalToLocal of h_{i+2} -> sIdx            (16-byte copies)
-//   q of h_{i+1}             -> sQ[(i+1) & 1]   (gathers through sIdx)
-// issued as one commit group at the start of iteration i; in FP32 the factors
-// of h_{i+1} -> sG, sW follow as the next group once iteration i's flux loop
-// is done with h_i's (FP64 reads its factors at the flux loop: staging them
-// would halve the resident blocks).  A thread gathers the nodes of the same
-// 16-byte index chunks it copies, so sIdx needs no barrier; q, the ids and the
-// factors are read by other threads after a wait and a barrier.  The q.Aq
-// partial reads q from sQ instead of gathering it again.
-template <int NQ>
-__global__ void __launch_bounds__(CubShape<NQ, CUB_STIFF>::THREADS, CubShape<NQ, CUB_STIFF>::MINB)
-ax_cub_pipe_kernel(int Nelements, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
-                   const CubReal* __restrict__ wJ, const CubReal* __restrict__ ggeo, CubReal lambda,
-                   const CubReal* __restrict__ q, CubReal* __restrict__ Aq, const int* __restrict__ skip,
-                   double* __restrict__ partials) {
-  constexpr int FORM = CUB_STIFF;
-  using F = CubReal;
-  using Sh = CubShape<NQ, FORM>;
-  static_assert(NQ % 2 == 0, "whole 16-byte index chunks");
-  constexpr bool STG = Sh::STAGE;   // FP32 stages the factors; FP64 reads them at the flux loop
-  constexpr int G = Sh::G, GP = Sh::GP, EPB = Sh::EPB, NP = Sh::NP, NQ2 = NQ * NQ;
-  constexpr int CH = NP / 4;   // 16-byte chunks of an element's GlobalToLocal
-  pdl_wait();
-  pdl_release();
-  if (skip && *skip) return;
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  F* const sbase = reinterpret_cast<F*>(smem_raw);
-  const int tx = threadIdx.x, ty = threadIdx.y, es = threadIdx.z;
-  const int tid = tx + G * (ty + G * es);
-  F* const U = sbase + (size_t)es * Sh::SLOTW;
-  F* const R = U + Sh::FIELD;
-  F* const S = R + Sh::FIELD;
-  F* const sG0 = reinterpret_cast<F*>(smem_raw + Sh::GOFF);
-  F* const sW0 = reinterpret_cast<F*>(smem_raw + Sh::WOFF);
-  int32_t* const sIdx = reinterpret_cast<int32_t*>(smem_raw + Sh::IOFF);
-  F* const sQ = reinterpret_cast<F*>(smem_raw + Sh::QOFF);
-  int32_t* const sEl = reinterpret_cast<int32_t*>(smem_raw + Sh::EOFF);
-
-  const int ngroups = (Nelements + EPB - 1) / EPB;
-  auto group = [&](int i) { return blockIdx.x + i * gridDim.x; };
-  // element ids of iteration i's group (-1 past the end) into sEl[i & 3]
-  auto issue_ids = [&](int i, bool async) {
-    if (tid < EPB) {
-      const int e = group(i) * EPB + tid;
-      int32_t* dst = sEl + (i & 3) * EPB + tid;
-      if (group(i) < ngroups && e < Nelements) {
-        if (async) cp_async4(dst, elementList + e);
-        else *dst = elementList[e];
-      } else {
-        *dst = -1;
-      }
-    }
-  };
-  // GlobalToLocal of iteration i's group into sIdx (ids in sEl[i & 3] visible)
-  auto issue_idx = [&](int i) {
-    for (int w = tid; w < EPB * CH; w += Sh::THREADS) {
-      const int s = w / CH, c = w - s * CH;
-      const int32_t e = sEl[(i & 3) * EPB + s];
-      if (e >= 0) cp_async16(sIdx + s * NP + 4 * c, G2L + (size_t)e * NP + 4 * c);
-    }
-  };
-  // q of iteration i's group into sQ[i & 1] through this thread's chunks of sIdx
-  auto issue_q = [&](int i) {
-    F* dstq = sQ + (size_t)(i & 1) * EPB * NP;
-    for (int w = tid; w < EPB * CH; w += Sh::THREADS) {
-      const int s = w / CH, c = w - s * CH;
-      const bool live = sEl[(i & 3) * EPB + s] >= 0;
-#pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int pos = s * NP + 4 * c + n;
-        const int32_t id = live ? sIdx[pos] : -1;
-        if (id < 0) dstq[pos] = F(0);
-        else if constexpr (sizeof(F) == 8) cp_async8(dstq + pos, q + id);
-        else cp_async4(dstq + pos, q + id);
-      }
-    }
-  };
-  // factors of iteration i's group into sG, sW
-  auto issue_factors = [&](int i) {
-    const int32_t e = sEl[(i & 3) * EPB + es];
-    if (e >= 0) {
-      const int tl = tx + G * ty;
-      const F* src = ggeo + 6 * (size_t)e * GP;   // 8-byte aligned: 24 bytes per point
-      F* sG = sG0 + (size_t)es * GP * 6;
-      for (int c = tl; c < GP * 3; c += G * G) cp_async8(sG + 2 * c, src + 2 * c);
-      const F* srcw = wJ + (size_t)e * GP;
-      F* sW = sW0 + (size_t)es * GP;
-      for (int c = tl; c < GP; c += G * G) cp_async4(sW + c, srcw + c);
-    }
-  };
-  struct PipeFactors {
-    CubStagedFactors<F> st;
-    const decltype(issue_factors)* next;
-    int i;
-    __device__ __forceinline__ void ready() const { cp_async_wait_group<1>(); }
-    __device__ __forceinline__ void released() const {
-      (*next)(i + 1);
-      cp_async_commit();
-    }
-    __device__ __forceinline__ void get(int pt, F (&g)[6], F& w) const { st.get(pt, g, w); }
-  };
-
-  // prologue: ids of iterations 0 and 1, indices of 0; then q of 0, indices
-  // of 1 and ids of 2 as one group, the factors of 0 as the next
-  issue_ids(0, false);
-  issue_ids(1, false);
   __syncthreads();
-  issue_idx(0);
-  cp_async_commit();
-  cp_async_wait_group<0>();   // this thread's index chunks
-  issue_q(0);
-  issue_idx(1);
-  issue_ids(2, true);
-  cp_async_commit();
-  if (STG) {
-    issue_factors(0);
-    cp_async_commit();
+  // along a, rows (j, c) = (lo, hi)
+  if (hi < NQ) {
+    F* const p = U + hi * PL + lo * RS;
+    F r[NQ];
+    cub_load<NQ, 1>(p, r);
+    cub_line<NQ, G, UN>(r, T, [&](int o, F x) { p[o] = x; });
   }
+  __syncthreads();
 
-  double pdot = 0.0;
-  for (int i = 0; group(i) < ngroups; ++i) {
-    if (STG) cp_async_wait_group<1>();   // all but the factors of this group
-    else cp_async_wait_group<0>();
-    __syncthreads();
-    const F* qg = sQ + (size_t)(i & 1) * EPB * NP + (size_t)es * NP;
-    const int32_t element = sEl[(i & 3) * EPB + es];
-    F qb[NQ];
-#pragma unroll
-    for (int b = 0; b < NQ; ++b) qb[b] = (tx < NQ && ty < NQ) ? qg[ty * NQ2 + b * NQ + tx] : F(0);
-    // the next groups' ids, indices and q
-    issue_q(i + 1);
-    issue_idx(i + 2);
-    issue_ids(i + 3, true);
-    cp_async_commit();
-
-    F qk[G], acc[G];
-    cub_interp<NQ, FORM>(qb, U, qk, tx, ty);
-    if constexpr (STG) {
-      const PipeFactors fac{CubStagedFactors<F>{sG0 + (size_t)es * GP * 6, sW0 + (size_t)es * GP}, &issue_factors,
-                            i};
-      cub_stiff<NQ, FORM>(qk, acc, U, R, S, tx, ty, lambda, fac);
-    } else {
-      const size_t e = element >= 0 ? (size_t)element : 0;
-      cub_stiff<NQ, FORM>(qk, acc, U, R, S, tx, ty, lambda, CubGlobalFactors<F>{ggeo + 6 * e * GP, wJ + e * GP});
+  F* const col = U + hi * RS + lo;            // column (i, j) = (lo, hi), this thread's own
+  if constexpr (FORM == CUB_MASS_AFFINE) {
+    if (t < G2 && valid) {
+      F r[NQ];
+      cub_load<NQ, PL>(col, r);
+      const F wa = __ldg(we);
+      cub_line<NQ, NQ, UN>(r, T, [&](int o, F x) {
+        const size_t l = lbase + o * NQ2 + t;
+        const F y = wa * x;
+        Aq[l] = y;
+        if (DOT) {
+          const int32_t id = __ldg(G2L + l);
+          pdot += (double)(id >= 0 ? __ldg(q + id) : F(0)) * (double)y;
+        }
+      });
     }
-    cub_project_ca<NQ, FORM>(acc, U, tx, ty);
-    if (tx < NQ && ty < NQ && element >= 0) {
-      F r[G];
+  } else if constexpr (FORM == CUB_MASS) {
+    // along c to the points, the weights, and back along c: row k of T serves both
+    if (t < G2) {
+      F r[NQ], a[NQ];
+      cub_load<NQ, PL>(col, r);
 #pragma unroll
-      for (int jj = 0; jj < G; ++jj) r[jj] = CUB_AT(U, ty, jj, tx);
-      const size_t lbase = (size_t)element * NP;
+      for (int n = 0; n < NQ; ++n) a[n] = 0;
+      const F* const wp = (valid ? we : wJ) + t;
+#pragma unroll UK
+      for (int k = 0; k < G; ++k) {
+        F o = 0, m[NQ];
 #pragma unroll
-      for (int b = 0; b < NQ; ++b) {
-        F t = 0;
+        for (int n = 0; n < NQ; ++n) {
+          m[n] = CUB_T(k, n);
+          o += m[n] * r[n];
+        }
+        const F w = __ldg(wp + k * G2);
+        if (DOT && valid) pdot += (double)(w * o) * (double)o;
+        o *= w;
 #pragma unroll
-        for (int jj = 0; jj < G; ++jj) t += CUB_T(jj, b) * r[jj];
-        Aq[lbase + ty * NQ2 + b * NQ + tx] = t;
-        if (partials) pdot += (double)qg[ty * NQ2 + b * NQ + tx] * (double)t;
+        for (int n = 0; n < NQ; ++n) a[n] += m[n] * o;
       }
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) col[n * PL] = a[n];
     }
+    __syncthreads();
+    if (hi < NQ) {   // along a, rows (j, c)
+      F* const p = U + hi * PL + lo * RS;
+      F s[G];
+      cub_load<G, 1>(p, s);
+      cub_line<G, NQ, UN>(s, Tt, [&](int o, F x) { p[o] = x; });
+    }
+    __syncthreads();
+    if (hn < NQ && valid) {   // along b, columns (a, c)
+      F s[G];
+      cub_load<G, RS>(U + hn * PL + ln, s);
+      cub_line<G, NQ, UN>(s, Tt, [&](int o, F x) { Aq[lbase + hn * NQ2 + o * NQ + ln] = x; });
+    }
+  } else {
+    if (t < G2) {   // along c to the points
+      F r[NQ];
+      cub_load<NQ, PL>(col, r);
+      cub_line<NQ, G, UN>(r, T, [&](int o, F x) { col[o * PL] = x; });
+    }
+    __syncthreads();
+    const int row = hi * PL + lo * RS, scol = hi * PL + lo;   // row (y, z), column (x, z) = (lo, hi)
+    if (t < G2) {
+      F r[G];
+      cub_load<G, 1>(U + row, r);
+      cub_line<G, G, UN>(r, D, [&](int o, F x) { R[row + o] = x; });
+      cub_load<G, RS>(U + scol, r);
+      cub_line<G, G, UN>(r, D, [&](int o, F x) { S[scol + o * RS] = x; });
+    }
+    __syncthreads();
+    if (t < G2) {   // the fluxes at the points of the column, the t-derivative and the t-part of the
+                    // divergence: row k of D serves both
+      F ga[6] = {0, 0, 0, 0, 0, 0}, wa = 0;
+      if (!Sh::CURVED && valid) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) ga[c] = __ldg(ge + c);
+        wa = __ldg(we);
+      }
+      const F* const gp = (valid ? ge : ggeo) + 6 * t;
+      const F* const wp = (valid ? we : wJ) + t;
+      F u[G], acc[G];
+      cub_load<G, PL>(col, u);
+#pragma unroll
+      for (int n = 0; n < G; ++n) acc[n] = 0;
+      F *pr = R + hi * RS + lo, *ps = S + hi * RS + lo;
+#pragma unroll UK
+      for (int k = 0; k < G; ++k) {
+        F g[6], w;
+        if (Sh::CURVED) {
+          const V2* gv = reinterpret_cast<const V2*>(gp + 6 * k * G2);
+          const V2 a0 = __ldg(gv), a1 = __ldg(gv + 1), a2 = __ldg(gv + 2);
+          g[0] = a0.x; g[1] = a0.y; g[2] = a1.x; g[3] = a1.y; g[4] = a2.x; g[5] = a2.y;
+          w = __ldg(wp + k * G2);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 6; ++c) g[c] = ga[c];
+          w = wa;
+        }
+        F m[G], d0 = 0, d1 = 0;   // two chains: the sum is on the critical path
+#pragma unroll
+        for (int n = 0; n < G; ++n) {
+          m[n] = CUB_D(k, n);
+          if (n & 1) d1 += m[n] * u[n];
+          else d0 += m[n] * u[n];
+        }
+        const F dr = pr[k * PL], ds = ps[k * PL], dt = d0 + d1, qk = col[k * PL];
+        const F fr = g[0] * dr + g[1] * ds + g[2] * dt, fs = g[1] * dr + g[3] * ds + g[4] * dt;
+        const F gt = g[2] * dr + g[4] * ds + g[5] * dt, mq = lambda * w * qk;
+        col[k * PL] = mq;
+        pr[k * PL] = fr;
+        ps[k * PL] = fs;
+        if (DOT && valid)   // products in FP64: their range is that of the squares
+          pdot += (double)dr * (double)fr + (double)ds * (double)fs + (double)dt * (double)gt + (double)mq * (double)qk;
+#pragma unroll
+        for (int n = 0; n < G; ++n) acc[n] += m[n] * gt;
+      }
+#pragma unroll
+      for (int n = 0; n < G; ++n) col[n * PL] += acc[n];
+    }
+    __syncthreads();
+    if (t < G2) {   // the r-part, added on rows
+      F r[G];
+      cub_load<G, 1>(R + row, r);
+      cub_line<G, G, UN>(r, Dt, [&](int o, F x) { U[row + o] += x; });
+    }
+    __syncthreads();
+    if (t < G2) {   // the s-part, added on columns (x, z), and the projection along b of the same columns
+      F r[G];
+      cub_load<G, RS>(S + scol, r);
+      cub_line<G, G, UN>(r, Dt, [&](int o, F x) { U[scol + o * RS] += x; });
+      cub_load<G, RS>(U + scol, r);
+      cub_line<G, NQ, UN>(r, Tt, [&](int o, F x) { U[scol + o * RS] = x; });
+    }
+    __syncthreads();
+    if (hi < NQ) {   // along c, columns (x, b) = (lo, hi)
+      F r[G];
+      cub_load<G, PL>(col, r);
+      cub_line<G, NQ, UN>(r, Tt, [&](int o, F x) { col[o * PL] = x; });
+    }
+    __syncthreads();
+    if (hn < NQ) {   // along a, rows (b, c) = (ln, hn)
+      F* const p = U + hn * PL + ln * RS;
+      F r[G];
+      cub_load<G, 1>(p, r);
+      cub_line<G, NQ, UN>(r, Tt, [&](int o, F x) { p[o] = x; });
+    }
+    __syncthreads();
+    if (valid && t < G2)   // out in node order: whole sectors
+      for (int n = t; n < NP; n += G2) {
+        const int c = n / NQ2, m = n - c * NQ2, b = m / NQ, a = m - b * NQ;
+        Aq[lbase + n] = U[c * PL + b * RS + a];
+      }
   }
-  cp_async_wait_all();   // nothing is left in flight (groups past the end issue no copies)
-  if (partials) {
-    static_assert(Sh::FIELDS >= sizeof(double) * Sh::THREADS, "scratch too small");
-    const double bs = fuse_block_sum(pdot, reinterpret_cast<double*>(sbase));
-    if (tid == 0) partials[blockIdx.x] = bs;
+  if (DOT) {
+    const double bs = fuse_block_sum(pdot, reinterpret_cast<double*>(smem_raw));
+    if (threadIdx.x == 0) partials[blockIdx.x] = bs;
   }
 }
-#undef CUB_AT
 #undef CUB_D
 #undef CUB_T
-
-// The pipelined stiffness kernel is the default where it applies;
-// BP_CUB_PIPE=0, read at every launch, keeps the one-element-per-slot kernel
-// (for comparisons and tests).
-static bool cub_pipe_enabled() {
-  const char* e = getenv("BP_CUB_PIPE");
-  return !(e && e[0] == '0');
-}
 
 // device address of the constant table on the current device
 static CubReal* cub_table_address() {
@@ -715,38 +413,13 @@ static int launch_cub_form(int32_t Nelements, int Nfields, const int32_t* elemen
   BP_TRY(const_slot_copy(tab + Sh::SLOT, o.T, sizeof(CubReal) * Sh::TSIZE, s));
   if (Sh::STIFF)
     BP_TRY(const_slot_copy(tab + Sh::SLOT + Sh::TSIZE, o.D, sizeof(CubReal) * Sh::DSIZE, s));
-  const dim3 block(Sh::G, Sh::G, Sh::EPB);
-  if constexpr (FORM == CUB_STIFF && NQ % 2 == 0 && Sh::PIPE_OK) {
-    if (Nfields == 1 && !(reinterpret_cast<uintptr_t>(G2L) & 15) && cub_pipe_enabled()) {
-      static DeviceOnce configured;
-      static int resident[kMaxDevices] = {};
-      BP_TRY(once_per_device(configured, []() -> int {
-        BP_CUDA_TRY(cudaFuncSetAttribute(ax_cub_pipe_kernel<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)Sh::PSMEM));
-        int dev = 0, nb = 0;
-        BP_TRY(current_device(&dev));
-        BP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ax_cub_pipe_kernel<NQ>, Sh::THREADS,
-                                                                  Sh::PSMEM));
-        resident[dev] = nb > 0 ? nb * sm_count() : 1;
-        return BP_SUCCESS;
-      }));
-      int dev = 0;
-      BP_TRY(current_device(&dev));
-      const int ngroups = (Nelements + Sh::EPB - 1) / Sh::EPB;
-      const dim3 grid(ngroups < resident[dev] ? ngroups : resident[dev]);
-      if (nblocks) *nblocks = (int)grid.x;
-      BP_CUDA_TRY(launch_pdl(ax_cub_pipe_kernel<NQ>, grid, block, Sh::PSMEM, s, Nelements, elementList, G2L, o.wJ,
-                             o.ggeo, lambda, q, Aq, skip, partials));
-      return BP_SUCCESS;
-    }
-  }
+  auto k = partials ? ax_cub_kernel<NQ, FORM, true> : ax_cub_kernel<NQ, FORM, false>;
   if (Sh::SMEM > 48 * 1024)
-    BP_CUDA_TRY(cudaFuncSetAttribute(ax_cub_kernel<NQ, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)Sh::SMEM));
-  const dim3 grid((Nelements + Sh::EPB - 1) / Sh::EPB);
+    BP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::SMEM));
+  const dim3 grid((unsigned)(((int64_t)Nelements * Nfields + Sh::EPB - 1) / Sh::EPB));
   if (nblocks) *nblocks = (int)grid.x;
-  BP_CUDA_TRY(launch_pdl(ax_cub_kernel<NQ, FORM>, grid, block, Sh::SMEM, s, Nelements, Nfields, elementList, G2L, o.wJ,
-                         o.ggeo, lambda, q, Aq, skip, partials));
+  BP_CUDA_TRY(launch_pdl(k, grid, dim3(Sh::THREADS), Sh::SMEM, s, Nelements, Nfields, elementList,
+                         G2L, o.wJ, o.ggeo, lambda, q, Aq, skip, partials));
   return BP_SUCCESS;
 }
 

@@ -1,6 +1,5 @@
 // FP32 instantiation of the over-integrated BP1-BP4 operators (mixed-precision CG).
 #define BP_CUB_REAL float
-#define BP_CUB_OUTER _Pragma("unroll")
 #include "bp_ax_cub.cuh"
 
 namespace bp {

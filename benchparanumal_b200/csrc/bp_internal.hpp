@@ -97,6 +97,15 @@ int const_slot_copy(void* dst, const void* src, size_t bytes, cudaStream_t s);
 bool pdl_enabled();
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The aligned whole 16-byte words of n values from p on, on their way to L2
+// (a hint: no wait, no result, nothing outside the n values).
+template <class F>
+__device__ __forceinline__ void l2_prefetch(const F* p, int n) {
+  const size_t a = (reinterpret_cast<size_t>(p) + 15) & ~(size_t)15;
+  const size_t e = reinterpret_cast<size_t>(p + n) & ~(size_t)15;
+  if (e > a)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
+}
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... KArgs, class... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {

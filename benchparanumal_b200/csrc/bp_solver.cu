@@ -1050,8 +1050,9 @@ int bp_solver_create(bp_mesh_t mesh, const bp_solver_desc_t* d, bp_solver_t* out
     if ((rc = S->partials.alloc((size_t)4 * reduction_blocks()))) break;
     if ((rc = S->counter.alloc(4))) break;
     // p.Ap epilogue of the element operator: one partial per block, at most
-    // one block per element
-    if ((rc = S->fuse_partials.alloc((size_t)mesh->E + 1))) break;
+    // one block per element and field (the simplex operator, which splits the
+    // rows of a small batch, two per SM)
+    if ((rc = S->fuse_partials.alloc((size_t)mesh->E * mesh->Nfields + 1 + 2 * sm_count()))) break;
     if ((rc = S->sc.alloc(1))) break;
     S->scal = S->sc.ptr;
     cudaError_t ce = cudaMemsetAsync(S->p.ptr, 0, sizeof(double) * S->N, s);
