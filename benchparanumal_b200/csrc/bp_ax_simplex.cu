@@ -123,6 +123,166 @@ ax_simplex_kernel(int Nelements, int Np, int groups, const int32_t* __restrict__
   }
 }
 
+// FP64 operator on the tensor cores (mma.sync m8n8k4 f64, the FP64 tensor
+// instruction; tcgen05 has no FP64 kind).  Per matrix X_c (S_ab.., MM) the
+// product P_c(n, e) = sum_k X_c(n, k) q(k, e) over M = Np nodes and N = elements,
+// then out = sum_c f_c(e) P_c: the reference's order, so each sum is Np terms
+// long (one sum over c and k together, the factors in the streamed operand, is
+// C Np terms and measured four times the rounding error).  A warp holds MT
+// m-tiles of 8 nodes by NT n-tiles of 8 elements; matrix fragments come from
+// global memory (node-fastest rows: 64 contiguous bytes per k, L1/L2 hits
+// after the first block) a group of KU k steps ahead of their use (an element
+// batch too small to fill the chip waits for L2 once per group), each serving
+// NT tiles; q comes from shared memory.  Rows past Np are computed on clamped
+// loads and not stored; k past Np multiplies zeros.  blockIdx.y takes every
+// gridDim.y-th set of rows.  Bound by the DMMA pipe and, at Np = 35, by the
+// gather ahead of it.  BK5 tetrahedra p=4 (93,600) 177 -> 122 us, p=7 (7,986)
+// 147 -> 84, p=15 (6) 590 -> 100; triangles p=15 (3,200) 69 -> 37 us, against
+// one thread per node on the FP64 cores.
+constexpr int kMmaWarps = 4;
+
+__device__ __forceinline__ void simplex_dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// words per element of the q tile: k padded to whole steps of 4, and 4 or 12
+// mod 16 so that the 4 x 4 fragment reads of a half-warp fall in distinct banks
+__host__ __device__ constexpr int simplex_kp(int Np) { return (Np + 3) / 4 * 4 + ((Np + 3) / 4 % 2 ? 0 : 4); }
+
+template <int C, int MT, int NT, bool DOT>
+__global__ void __launch_bounds__(kMmaWarps * 32)
+ax_simplex_mma_kernel(int Nelements, int Np, int wm, const int32_t* __restrict__ elementList,
+                      const int32_t* __restrict__ G2L, const double* __restrict__ wJ,
+                      const double* __restrict__ ggeo, const double* __restrict__ S, const double* __restrict__ MM,
+                      double lambda, const double* __restrict__ q, double* __restrict__ Aq,
+                      const int* __restrict__ skip, double* __restrict__ partials) {
+  pdl_wait();
+  pdl_release();
+  if (skip && *skip) return;
+  extern __shared__ __align__(16) double s_raw[];
+  const int KP = simplex_kp(Np), KT = (Np + 3) / 4;
+  const int wn = kMmaWarps / wm;                 // warps along the elements
+  const int EB = wn * NT * 8;                    // elements per block
+  double* const s_q = s_raw;                     // [EB][KP]
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, g = lane >> 2, t4 = lane & 3;
+  const int e0 = blockIdx.x * EB;
+  // gather in batches: the index loads of a batch in flight together, then its values
+  constexpr int GB = 6;
+  for (int i0 = t; i0 < EB * KP; i0 += GB * kMmaWarps * 32) {
+    int32_t id[GB];
+#pragma unroll
+    for (int u = 0; u < GB; ++u) {
+      const int i = i0 + u * kMmaWarps * 32, j = i / KP, m = i - j * KP;
+      id[u] = i < EB * KP && m < Np && e0 + j < Nelements ? G2L[(size_t)elementList[e0 + j] * Np + m] : -1;
+    }
+    double v[GB];
+#pragma unroll
+    for (int u = 0; u < GB; ++u) v[u] = id[u] >= 0 ? q[id[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < GB; ++u)
+      if (i0 + u * kMmaWarps * 32 < EB * KP) s_q[i0 + u * kMmaWarps * 32] = v[u];
+  }
+  __syncthreads();
+  const int mw = w % wm, eb = (w / wm) * NT * 8;   // this warp's row of m-sets and first element
+  // the elements of this lane's accumulator columns nt*8 + 2 t4 + h (-1: none)
+  int el[NT][2];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int eidx = e0 + eb + nt * 8 + 2 * t4 + h;
+      el[nt][h] = eidx < Nelements ? elementList[eidx] : -1;
+    }
+  const size_t NP2 = (size_t)Np * Np;
+  const double* const sq = s_q + (size_t)(eb + g) * KP + t4;
+  double pdot = 0.0;
+  for (int m0 = (blockIdx.y * wm + mw) * MT * 8; m0 < Np; m0 += gridDim.y * wm * MT * 8) {
+    double tot[MT][NT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) tot[mt][nt][0] = tot[mt][nt][1] = 0.0;
+    int row[MT];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) row[mt] = min(m0 + mt * 8 + g, Np - 1) + t4 * Np;
+    // fragments of the matrix X at the KU k steps from kt on (past the end: zeros)
+    constexpr int KU = NT == 2 ? 1 : 4;
+    auto load_a = [&](const double* X, int kt, double (&a)[KU][MT]) {
+#pragma unroll
+      for (int u = 0; u < KU; ++u)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+          a[u][mt] = (kt + u) * 4 + t4 < Np ? __ldg(X + (size_t)(kt + u) * 4 * Np + row[mt]) : 0.0;
+    };
+    double nxt[KU][MT];
+    load_a(S, 0, nxt);
+#pragma unroll 1
+    for (int c = 0; c < C; ++c) {
+      const double* const X = c < C - 1 ? S + c * NP2 : MM;
+      const double* const Xn = c + 1 < C - 1 ? X + NP2 : MM;   // the next matrix
+      double acc[MT][NT][2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
+#pragma unroll(KU == 1 ? 2 : 1)
+      for (int kt = 0; kt < KT; kt += KU) {
+        double a[KU][MT];
+#pragma unroll
+        for (int u = 0; u < KU; ++u)
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) a[u][mt] = nxt[u][mt];
+        const bool last = kt + KU >= KT;
+        load_a(last ? Xn : X, last ? 0 : kt + KU, nxt);
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+          if (u > 0 && kt + u >= KT) break;
+          double b[NT];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) b[nt] = sq[nt * 8 * KP + (kt + u) * 4];
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) simplex_dmma(acc[mt][nt], a[u][mt], b[nt]);
+        }
+      }
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const size_t e = el[nt][h] < 0 ? 0 : el[nt][h];
+          const double f = el[nt][h] < 0 ? 0.0 : c < C - 1 ? __ldg(ggeo + (C - 1) * e + c) : __ldg(wJ + e) * lambda;
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) tot[mt][nt][h] += f * acc[mt][nt][h];
+        }
+    }
+    // accumulator of lane (g, t4): node m0 + mt*8 + g, elements nt*8 + 2 t4 + {0, 1}
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (el[nt][h] >= 0) {
+          const int j = eb + nt * 8 + 2 * t4 + h;
+          double* const o = Aq + (size_t)el[nt][h] * Np;
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            const int n = m0 + mt * 8 + g;
+            if (n < Np) {
+              o[n] = tot[mt][nt][h];
+              if (DOT) pdot += s_q[(size_t)j * KP + n] * tot[mt][nt][h];
+            }
+          }
+        }
+      }
+  }
+  if (DOT) {
+    const double bs = fuse_block_sum(pdot, s_raw);
+    if (t == 0) partials[blockIdx.y * gridDim.x + blockIdx.x] = bs;
+  }
+}
+
 // b_e = J_e MM f_e with f scattered through GlobalToLocal (masked nodes 0)
 __global__ void __launch_bounds__(kTriThreads + 32)
 tri_mass_local_kernel(int Nelements, int Np, int epb, const int32_t* __restrict__ G2L,
@@ -206,6 +366,74 @@ int launch_rhs_analytic_simplex(int dim, int N, int32_t Nelements, const double*
   return BP_SUCCESS;
 }
 
+// Warps along the nodes (wm of kMmaWarps; the others along the elements),
+// m-tiles and n-tiles per warp, blocks along the nodes.
+struct SimplexMmaPlan {
+  int mt, nt, wm, gy;
+  int eb() const { return kMmaWarps / wm * nt * 8; }
+  size_t smem(int Np) const { return sizeof(double) * (size_t)eb() * simplex_kp(Np); }
+};
+
+// The plan with the least estimated time: the rounds of row sets a warp runs,
+// times the tile products, fragment loads and latency of a k step, times the
+// blocks beyond what three per SM hold.  A batch that leaves the chip idle
+// spreads its rows over blockIdx.y, to at most about two blocks per SM.
+static SimplexMmaPlan simplex_mma_plan(int Np, int32_t E, int sms) {
+  const int tiles = (Np + 7) / 8;
+  SimplexMmaPlan best{1, 1, 1, 1};
+  double cost = 1e300;
+  for (int nt = 2; nt >= 1; --nt)
+    for (int wm = 1; wm <= kMmaWarps; wm *= 2)
+      for (int mt = 1; mt <= 5; ++mt) {
+        SimplexMmaPlan p{mt, nt, wm, 1};
+        if (p.smem(Np) > 48 * 1024 && (nt > 1 || wm < kMmaWarps)) continue;
+        const int sets = (tiles + mt * wm - 1) / (mt * wm);
+        const int bx = (E + p.eb() - 1) / p.eb();
+        p.gy = std::max(1, std::min(sets, 2 * sms / bx));
+        const int rounds = (sets + p.gy - 1) / p.gy;
+        const double waves = (double)bx * p.gy / (3 * sms);
+        const double c = std::max(waves, 1.0) * rounds * (mt * nt + 0.6 * mt + 0.3 * nt + 1.5);
+        if (c < cost) {
+          cost = c;
+          best = p;
+        }
+      }
+  return best;
+}
+
+template <int C, int MT, int NT>
+static int launch_simplex_mma(const SimplexMmaPlan& p, int Np, int32_t E, const int32_t* elementList,
+                              const int32_t* G2L, const double* wJ, const double* ggeo, const double* S,
+                              const double* MM, double lambda, const double* q, double* Aq, const int* skip,
+                              cudaStream_t s, double* partials, int* nblocks) {
+  const dim3 grid((E + p.eb() - 1) / p.eb(), p.gy);
+  if (nblocks) *nblocks = (int)(grid.x * grid.y);
+  const size_t smem = p.smem(Np);
+  auto k = partials ? ax_simplex_mma_kernel<C, MT, NT, true> : ax_simplex_mma_kernel<C, MT, NT, false>;
+  if (smem > 48 * 1024) BP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  BP_CUDA_TRY(launch_pdl(k, grid, kMmaWarps * 32, smem, s, (int)E, Np, p.wm, elementList, G2L, wJ, ggeo, S, MM, lambda,
+                         q, Aq, skip, partials));
+  return BP_SUCCESS;
+}
+
+template <int C>
+static int launch_ax_simplex_mma(int N, int32_t E, const int32_t* elementList, const int32_t* G2L, const double* wJ,
+                                 const double* ggeo, const double* S, const double* MM, double lambda,
+                                 const double* q, double* Aq, const int* skip, cudaStream_t s, double* partials,
+                                 int* nblocks) {
+  const int Np = simplex_np(C == 4 ? 2 : 3, N);
+  const SimplexMmaPlan p = simplex_mma_plan(Np, E, sm_count());
+#define BP_SIMPLEX_MMA(MT, NT)                                                                                     \
+  if (p.mt == MT && p.nt == NT)                                                                                    \
+    return launch_simplex_mma<C, MT, NT>(p, Np, E, elementList, G2L, wJ, ggeo, S, MM, lambda, q, Aq, skip, s, partials, \
+                                         nblocks);
+#define BP_SIMPLEX_MMA_NT(MT) BP_SIMPLEX_MMA(MT, 1) BP_SIMPLEX_MMA(MT, 2)
+  BP_SIMPLEX_MMA_NT(1) BP_SIMPLEX_MMA_NT(2) BP_SIMPLEX_MMA_NT(3) BP_SIMPLEX_MMA_NT(4) BP_SIMPLEX_MMA_NT(5)
+#undef BP_SIMPLEX_MMA_NT
+#undef BP_SIMPLEX_MMA
+  return fail(BP_ERROR_ARG, "simplex operator: no tile shape");
+}
+
 template <class F, int NSM>
 static int launch_ax_simplex_t(int N, int32_t Nelements, const int32_t* elementList, const int32_t* G2L, const F* wJ,
                                const F* ggeo, const F* S, const F* MM, F lambda, const F* q, F* Aq, const int* skip,
@@ -214,6 +442,12 @@ static int launch_ax_simplex_t(int N, int32_t Nelements, const int32_t* elementL
   if (N < 1 || N > 15) return fail(BP_ERROR_ARG, "simplex operator: degree N must be in 1..15");
   if (Nelements == 0) return BP_SUCCESS;
   const int Np = simplex_np(NSM == 3 ? 2 : 3, N);
+  // an element of less than one m-tile of nodes is mostly padding there (triangles
+  // p=1: 42 us scalar against 81; p=2 and tetrahedra p=1 the same in both)
+  if constexpr (sizeof(F) == 8)
+    if (Np >= 8)
+      return launch_ax_simplex_mma<NSM + 1>(N, Nelements, elementList, G2L, wJ, ggeo, S, MM, lambda, q, Aq, skip, s,
+                                            partials, nblocks);
   int groups = 0, threads = 0;
   tri_shape(Np, &groups, &threads);
   const int slots = groups * kTriElems;
