@@ -1,6 +1,5 @@
 // FP32 instantiation of the line-per-thread BP5/BP6 element operator (mixed-precision CG).
 #define BP_LINE_REAL float
-#define BP_LINE_UNROLL_MAX 16
 #include "bp_ax_line.cuh"
 #include "bp_cg_persist.cuh"
 
@@ -13,7 +12,7 @@ struct LineStepOp {
   static constexpr int THREADS = LineShape<NQ, T>::THREADS;
   static constexpr int MINB = LineMinBlocks<NQ, T>::V;
   static __device__ __forceinline__ void run(int blk, const GrpStepArgs& a, unsigned char* smem) {
-    ax_line_body<NQ, AFFINE, T>(blk, a.nblk_op, a.Nelements, 1, a.elementList, a.G2L, a.wJ, a.ggeo, a.gllw,
+    ax_line_body<NQ, AFFINE, T>(blk, a.nblk_op, a.Nelements, a.elementList, a.G2L, a.wJ, a.ggeo, a.gllw,
                                 a.lambda, reinterpret_cast<const T*>(a.p), reinterpret_cast<T*>(a.AqL), a.parts,
                                 smem);
   }
@@ -29,7 +28,7 @@ int launch_step_line_nq(const bp_ax_desc_t& d, GrpStepArgs a, int grid_cap, cuda
   if (d.affine)
     BP_TRY(const_slot_copy(tab + Sh::SLOT + NQ * NQ, a.gllw, sizeof(float) * NQ, s));
   a.nblk_op = (a.Nelements + Sh::EPB - 1) / Sh::EPB;
-  const dim3 block(NQ, NQ, Sh::EPB);
+  const dim3 block(Sh::THREADS);
   if (d.affine) return launch_grp_step_kernel<PK, LineStepOp<NQ, true, T>>(a, block, Sh::smem(), grid_cap, s);
   return launch_grp_step_kernel<PK, LineStepOp<NQ, false, T>>(a, block, Sh::smem(), grid_cap, s);
 }

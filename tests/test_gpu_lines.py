@@ -1,0 +1,63 @@
+"""The line forms of the BP5/BP6 operators where a block or warp serves several
+(element, field) slots: permuted partial element lists on Hex3D (one value per
+node and four packed), Quad2D on both sides of the rule that picks its form,
+and the simplex operator's row split, against the FP64 oracle.
+
+1e-12 relative in FP64 as elsewhere (sums of at most 136 terms on the simplex,
+16 per 1D step); 2e-5 in FP32, the bar of the other FP32 operators."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float(np.max(np.abs(a - b)) / max(np.max(np.abs(b)), 1e-300))
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 5, 6, 7, 9, 12, 15])
+@pytest.mark.parametrize("affine,nf", [(False, 1), (True, 1), (False, 3), (True, 3)])
+def test_hex_permuted_subset(gpu, oracle, monkeypatch, N, affine, nf):
+    monkeypatch.setenv("BP_AX_VARIANT", "line")
+    om = oracle.Mesh(3, 2, 2, N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1)
+    gm = gpu.Mesh(3, 2, 2, N=N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1)
+    q = 2 * oracle.random(5, om.Ngather) - 1
+    want = om.ax(q).reshape(gm.E, -1)
+    els = np.array([10, 3, 7, 0, 11], np.int32)
+    dq, dA = gpu.DeviceBuffer.from_host(q), gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
+    de = gpu.DeviceBuffer.from_host(els)
+    gpu.ax_hex3d(gm, dq, dA, elementList=de.ptr, Nelements=els.size)
+    got = dA.download().reshape(gm.E, -1)
+    assert np.all(np.isnan(got[np.setdiff1d(np.arange(gm.E), els)]))
+    assert _rel(got[els], want[els]) < 1e-12
+
+
+@pytest.mark.parametrize("N", [1, 2, 3, 4, 5, 6, 7, 8, 10])
+def test_packed_lines(gpu, oracle, monkeypatch, N):
+    monkeypatch.setenv("BP_AX_VARIANT", "line")
+    om, gm = oracle.Mesh(3, 3, 2, N, pert=0.1), gpu.Mesh(3, 3, 2, N=N, pert=0.1)
+    v, ng = gm.view, gm.E * gm.Np
+    ops = {}
+    for name, n in (("wJ", ng), ("ggeo", 6 * ng), ("gllw", gm.Nq), ("D", gm.Nq ** 2)):
+        ops[name] = gpu.DeviceBuffer(n, np.float32)
+        gpu.convert_f64_f32(getattr(v, name), n, ops[name])
+    q = np.stack([2 * oracle.random(k, om.Ngather) - 1 for k in range(4)], 1).astype(np.float32)
+    dq = gpu.DeviceBuffer.from_host(q)
+    dA = gpu.DeviceBuffer.from_host(np.full(4 * gm.NL, np.nan, np.float32))
+    gpu.ax_hex3d_f32_multi(gm, 4, dq, dA, ops)
+    got = dA.download().reshape(-1, 4).astype(np.float64)
+    for k in range(4):
+        assert _rel(got[:, k], om.ax(q[:, k].astype(np.float64))) < 2e-5
+
+
+# 3 x 2 elements: the node form above Nq = 4; 40 x 31: the line form up to Nq = 16
+@pytest.mark.parametrize("nx,ny", [(3, 2), (40, 31)])
+@pytest.mark.parametrize("N", [1, 4, 6, 9, 15])
+@pytest.mark.parametrize("affine,nf", [(False, 1), (True, 1), (False, 2), (True, 2)])
+def test_quad_forms(gpu, oracle, nx, ny, N, affine, nf):
+    om = oracle.Mesh(nx, ny, 0, N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1, dim=2)
+    gm = gpu.Mesh(nx, ny, 1, N=N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1, dim=2)
+    q = 2 * oracle.random(5, om.Ngather) - 1
+    dq, dA = gpu.DeviceBuffer.from_host(q), gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
+    gpu.ax_hex3d(gm, dq, dA)
+    assert _rel(dA.download(), om.ax(q)) < 1e-12
