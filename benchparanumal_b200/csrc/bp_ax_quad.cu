@@ -5,13 +5,11 @@
 //   (ur, us) = (Dr, Ds) q
 // (okl/bp5AxQuad2D.okl, okl/bp5AxAffineQuad2D.okl, okl/bp6AxQuad2D.okl with
 // Nfields = dim = 2).  Stored factors carry the GLL weights; affine factors are
-// per element and the weights w_i w_j are applied here.  One thread per node
-// (i, j) of an element slot, EPB element slots per block; q, the fluxes and D
-// go through shared memory (rows padded by one word), which the Nq^2 nodes of
-// a 2D element fill in one pass.
+// per element and the weights w_i w_j are applied here.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "bp_cg_device.cuh"
 #include "bp_internal.hpp"
@@ -19,8 +17,166 @@
 namespace bp {
 namespace {
 
+// One warp serves SPW element(-field)s of NQ lines each; a thread owns column x
+// of its element in registers (q, then the result) and row y of the r-steps.
+// Shared memory carries what crosses between rows and columns (ten accesses of
+// a value per node); D and its transpose are read as warp-uniform pairs
+// (broadcasts), and a row of D serves both the s-derivative and the s-part of
+// the divergence.  Warps are independent: no block barrier after D is there.
+//
+// Before, one thread per node read a row and a column of q, of the r- and
+// s-fluxes and of D for every node (66 shared-memory accesses; 93% of the L1
+// pipe, 0.45 of HBM); affine factors took a column form with block barriers.
+// BK5 p=7 700x500 curved: 373 -> 252 us.
 template <int NQ>
 struct QuadShape {
+  static constexpr int SPW = 32 / NQ;                     // element(-field)s per warp
+  static constexpr int WARPS = 4, THREADS = 32 * WARPS;
+  static constexpr int EPB = SPW * WARPS;
+  static constexpr int RS = NQ % 2 ? NQ : NQ + 1;         // odd row stride: rows fall in distinct banks
+  static constexpr int NP = NQ * NQ;
+  static constexpr int DS = NQ + NQ % 2;                  // rows of D padded to whole pairs
+};
+
+// sum of the NQ products d[n] r[n], d read in pairs
+template <int NQ, class F>
+__device__ __forceinline__ F quad_dot(const F* d, const F (&r)[NQ]) {
+  using V2 = typename std::conditional<sizeof(F) == 8, double2, float2>::type;
+  F a = 0;
+#pragma unroll
+  for (int n = 0; n + 1 < NQ; n += 2) {
+    const V2 v = *reinterpret_cast<const V2*>(d + n);
+    a += v.x * r[n];
+    a += v.y * r[n + 1];
+  }
+  if (NQ % 2) a += d[NQ - 1] * r[NQ - 1];
+  return a;
+}
+
+template <int NQ, bool AFFINE, bool DOT, class F>
+__global__ void __launch_bounds__(QuadShape<NQ>::THREADS)
+ax_quad_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
+               const F* __restrict__ wJ, const F* __restrict__ ggeo, const F* __restrict__ gllw,
+               const F* __restrict__ Dg, F lambda, const F* __restrict__ q, F* __restrict__ Aq,
+               const int* __restrict__ skip, CgFuse fuse) {
+  if (skip && *skip) return;
+  using Sh = QuadShape<NQ>;
+  constexpr int RS = Sh::RS, NP = Sh::NP, DS = Sh::DS, SPW = Sh::SPW;
+  __shared__ __align__(16) F s_D[NQ * DS];    // row o of D
+  __shared__ __align__(16) F s_Dt[NQ * DS];   // row o of D^T
+  __shared__ F s_U[Sh::EPB][NQ * RS];
+  __shared__ F s_R[Sh::EPB][NQ * RS];
+  __shared__ double s_red[Sh::WARPS];
+  for (int n = threadIdx.x; n < NP; n += Sh::THREADS) {
+    const F d = Dg[n];
+    s_D[n / NQ * DS + n % NQ] = d;
+    s_Dt[n % NQ * DS + n / NQ] = d;
+  }
+  const int lane = threadIdx.x & 31, sl = lane / NQ;
+  const bool on = sl < SPW;                               // the last lanes own no line
+  const int slot = (threadIdx.x >> 5) * SPW + (on ? sl : 0), x = on ? lane - sl * NQ : 0;
+  const int v = blockIdx.x * Sh::EPB + slot;              // element-major (element, field)
+  const bool valid = on && v < Nelements * Nfields;
+  const int eidx = Nfields == 1 ? v : v / Nfields, f = v - eidx * Nfields;
+  const int e = valid ? elementList[eidx] : 0;
+  const size_t lbase = ((size_t)e * Nfields + f) * NP;
+  const F* const ge = ggeo + 3 * (size_t)e * (AFFINE ? 1 : NP);
+  const F* const we = wJ + (size_t)e * (AFFINE ? 1 : NP);
+  if (!AFFINE && NQ > 4 && valid && x == 0) {   // (smaller elements: more requests than they save)
+    l2_prefetch(ge, 3 * NP);
+    l2_prefetch(we, NP);
+  }
+  F* const U = s_U[slot];
+  F* const R = s_R[slot];
+  F u[NQ];   // column x
+  {
+    int32_t id[NQ];
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) id[j] = valid ? __ldg(G2L + lbase + j * NQ + x) : -1;
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) u[j] = id[j] >= 0 ? __ldg(q + id[j]) : F(0);
+  }
+  if (on) {
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) U[j * RS + x] = u[j];
+  }
+  __syncthreads();   // D is there
+  double pdot = 0.0;
+  if (on) {   // r-derivative on row x
+    F r[NQ];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) r[n] = U[x * RS + n];
+#pragma unroll
+    for (int o = 0; o < NQ; ++o) R[x * RS + o] = quad_dot<NQ>(s_D + o * DS, r);
+  }
+  __syncwarp();
+  if (on) {   // column x: s-derivative, fluxes, s-part of the divergence
+    F ga[3] = {0, 0, 0}, wa = 0;
+    if (AFFINE && valid) {
+      const F wx = __ldg(gllw + x);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ga[c] = __ldg(ge + c) * wx;
+      wa = __ldg(we) * wx;
+    }
+    const F* const gp = (valid ? ge : ggeo) + 3 * x;
+    const F* const wp = (valid ? we : wJ) + x;
+    F acc[NQ];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) acc[n] = 0;
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      F g0, g1, g2, w;
+      if (AFFINE) {
+        const F wj = __ldg(gllw + j);
+        g0 = ga[0] * wj; g1 = ga[1] * wj; g2 = ga[2] * wj;
+        w = wa * wj;
+      } else {
+        g0 = __ldg(gp + 3 * j * NQ); g1 = __ldg(gp + 3 * j * NQ + 1); g2 = __ldg(gp + 3 * j * NQ + 2);
+        w = __ldg(wp + j * NQ);
+      }
+      const F ur = R[j * RS + x], us = quad_dot<NQ>(s_D + j * DS, u);
+      const F fr = g0 * ur + g1 * us, fs = g1 * ur + g2 * us, mq = lambda * w * u[j];
+      R[j * RS + x] = fr;
+      acc[j] += mq;
+      if (DOT && valid)
+        pdot += (double)ur * (double)fr + (double)us * (double)fs + (double)mq * (double)u[j];
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) acc[n] += s_D[j * DS + n] * fs;
+    }
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) U[n * RS + x] = acc[n];
+  }
+  __syncwarp();
+  if (on) {   // r-part of the divergence on row x
+    F r[NQ];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) r[n] = R[x * RS + n];
+#pragma unroll
+    for (int o = 0; o < NQ; ++o) U[x * RS + o] += quad_dot<NQ>(s_Dt + o * DS, r);
+  }
+  __syncwarp();
+  if (valid) {   // out by columns: whole sectors
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) Aq[lbase + j * NQ + x] = U[j * RS + x];
+  }
+  if (DOT) {
+    pdot = warp_tree_sum(pdot);
+    if (lane == 0) s_red[threadIdx.x >> 5] = pdot;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double r = 0.0;
+      for (int w = 0; w < Sh::WARPS; ++w) r += s_red[w];
+      fuse.partials[blockIdx.x] = r;
+    }
+  }
+}
+
+// Node form, for meshes too small to fill the chip with warps: one thread per
+// node, so an element takes Nq dependent steps where the line form takes Nq^2
+// per thread (BK5 p=15, 42 elements: 6.7 us against 12; 100,000 elements 39
+// against 60 us the other way).
+template <int NQ>
+struct QuadNodeShape {
   static constexpr int EPB0 = 256 / (NQ * NQ);
   static constexpr int EPB = EPB0 < 1 ? 1 : (EPB0 > 16 ? 16 : EPB0);   // element slots per block
   static constexpr int RS = NQ + 1;                                     // padded row
@@ -28,13 +184,13 @@ struct QuadShape {
 };
 
 template <int NQ, int NF, bool AFFINE, bool DOT, class F>
-__global__ void __launch_bounds__(QuadShape<NQ>::THREADS)
-ax_quad_kernel(int Nelements, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
+__global__ void __launch_bounds__(QuadNodeShape<NQ>::THREADS)
+ax_quad_node_kernel(int Nelements, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
                const F* __restrict__ wJ, const F* __restrict__ ggeo, const F* __restrict__ gllw,
                const F* __restrict__ Dg, F lambda, const F* __restrict__ q, F* __restrict__ Aq,
                const int* __restrict__ skip, CgFuse fuse) {
   if (skip && *skip) return;
-  using Sh = QuadShape<NQ>;
+  using Sh = QuadNodeShape<NQ>;
   constexpr int EPB = Sh::EPB, RS = Sh::RS, NP = NQ * NQ;
   __shared__ F s_D[NQ][RS];
   __shared__ F s_w[NQ];
@@ -99,156 +255,32 @@ ax_quad_kernel(int Nelements, const int32_t* __restrict__ elementList, const int
   if (DOT) fuse_pap(pdot, fuse, s_red);
 }
 
-// Column form (affine factors, NQ <= kQuadColMax): one thread per column i of
-// an element, holding the column's q values and s-fluxes in registers and row
-// and column i of D; shared memory carries only what crosses columns (the rows
-// of q and of the r-flux), and the other reads of D use a slice index that is
-// the same for every lane (broadcasts).  The sums run in the node form's
-// order.  Measured on 800x800 boxes (the same box, two alternating runs): BK5
-// affine p=3 3.59 -> 4.96, p=5 4.34 -> 5.10, p=7 4.77 -> 5.87, p=9 4.61 ->
-// 5.04 TFLOP/s, 100 CG iterations at p=7 123.0 -> 107.1 ms; with stored
-// factors it lost (p=7 3.03 -> 2.48 TB/s: 88-102 registers leave two blocks
-// per SM to wait on the per-node factor loads), so those keep the node form;
-// staging each slot's stored factors in shared memory first (coalesced loads,
-// 12 slots per block for the space, 142 registers) was slower still: p=7 1.55
-// TB/s.
-constexpr int kQuadColMax = 10;
-
-template <int NQ>
-struct QuadColShape {
-  static constexpr int EPB = (NQ <= 8 ? 256 : 160) / NQ;   // element slots per block
-  static constexpr int RS = NQ + 1;
-  static constexpr int THREADS = NQ * EPB;
-};
-
-template <int NQ, int NF, bool AFFINE, bool DOT, class F>
-__global__ void __launch_bounds__(QuadColShape<NQ>::THREADS)
-ax_quad_col_kernel(int Nelements, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
-                   const F* __restrict__ wJ, const F* __restrict__ ggeo, const F* __restrict__ gllw,
-                   const F* __restrict__ Dg, F lambda, const F* __restrict__ q, F* __restrict__ Aq,
-                   const int* __restrict__ skip, CgFuse fuse) {
-  if (skip && *skip) return;
-  using Sh = QuadColShape<NQ>;
-  constexpr int EPB = Sh::EPB, RS = Sh::RS, NP = NQ * NQ;
-  __shared__ F s_D[NQ][NQ];
-  __shared__ F s_w[NQ];
-  __shared__ F s_q[EPB][NQ][RS];   // rows of q (one field at a time)
-  __shared__ F s_r[EPB][NQ][RS];   // rows of the r-flux
-  __shared__ double s_red[Sh::THREADS];
-
-  const int i = threadIdx.x, es = threadIdx.y;
-  const int t = i + NQ * es;
-  const int eidx = blockIdx.x * EPB + es;
-  const bool active = eidx < Nelements;
-  const int e = active ? elementList[eidx] : 0;
-  for (int n = t; n < NP; n += Sh::THREADS) s_D[n / NQ][n % NQ] = Dg[n];
-  if (AFFINE && t < NQ) s_w[t] = gllw[t];
-  __syncthreads();
-  F Di[NQ], Dci[NQ];   // row i and column i of D
-#pragma unroll
-  for (int m = 0; m < NQ; ++m) {
-    Di[m] = s_D[i][m];
-    Dci[m] = s_D[m][i];
-  }
-  F A00 = 0, A01 = 0, A11 = 0, AJ = 0;   // affine factors (the weights w_i w_j applied per node)
-  if (AFFINE && active) {
-    A00 = ggeo[3 * (size_t)e + 0];
-    A01 = ggeo[3 * (size_t)e + 1];
-    A11 = ggeo[3 * (size_t)e + 2];
-    AJ = wJ[e];
-  }
-  double pdot = 0.0;
-#pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    const size_t lb = ((size_t)e * NF + f) * NP + i;
-    F qc[NQ];
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-      const int32_t id = active ? G2L[lb + j * NQ] : -1;
-      qc[j] = (id != -1) ? q[id] : F(0);
-      s_q[es][j][i] = qc[j];
-    }
-    __syncthreads();
-    F fs[NQ];
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-      F ur = 0, us = 0;
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) {
-        ur += Di[m] * s_q[es][j][m];
-        us += s_D[j][m] * qc[m];
-      }
-      F G00, G01, G11;
-      if (AFFINE) {
-        const F w = s_w[i] * s_w[j];
-        G00 = A00 * w;
-        G01 = A01 * w;
-        G11 = A11 * w;
-      } else {
-        const size_t gb = (size_t)e * NP + j * NQ + i;
-        G00 = active ? ggeo[3 * gb + 0] : F(0);
-        G01 = active ? ggeo[3 * gb + 1] : F(0);
-        G11 = active ? ggeo[3 * gb + 2] : F(0);
-      }
-      s_r[es][j][i] = G00 * ur + G01 * us;
-      fs[j] = G01 * ur + G11 * us;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) {
-      const F GwJ = AFFINE ? AJ * (s_w[i] * s_w[j]) : (active ? wJ[(size_t)e * NP + j * NQ + i] : F(0));
-      F ap = qc[j] * lambda * GwJ;
-#pragma unroll
-      for (int m = 0; m < NQ; ++m) {
-        ap += Dci[m] * s_r[es][j][m];
-        ap += s_D[m][j] * fs[m];
-      }
-      if (active) Aq[lb + j * NQ] = ap;
-      if (DOT) pdot += (double)qc[j] * (double)ap;
-    }
-    if (NF > 1) __syncthreads();   // the next field reuses s_q and s_r
-  }
-  if (DOT) fuse_pap(pdot, fuse, s_red);
-}
-
-// element slots per block of the form that runs (the column form exists for NQ <= kQuadColMax)
-template <int NQ>
-int quad_epb(bool col) {
-  if constexpr (NQ <= kQuadColMax)
-    return col ? QuadColShape<NQ>::EPB : QuadShape<NQ>::EPB;
-  else
-    return QuadShape<NQ>::EPB;
-}
-
 template <int NQ, class F>
 static int launch_quad_nq(const bp_ax_desc_t& d, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                           const F* wJ, const F* ggeo, const F* gllw, const F* D, F lambda, const F* q, F* Aq,
                           const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks) {
-  constexpr bool COL = NQ <= kQuadColMax;
-  const bool col = COL && d.affine;
-  const int epb = quad_epb<NQ>(col);
-  const dim3 block = col ? dim3(NQ, epb) : dim3(NQ, NQ, epb);
-  const dim3 grid((Nelements + epb - 1) / epb);
-  if (nblocks) *nblocks = (int)grid.x;
+  using Sh = QuadShape<NQ>;
   const CgFuse Fz = fuse ? *fuse : CgFuse{};
-#define BP_QUAD(NF, AFF, DOT)                                                                                        \
-  do {                                                                                                               \
-    if constexpr (COL && AFF)                                                                                        \
-      ax_quad_col_kernel<NQ, NF, AFF, DOT, F><<<grid, block, 0, s>>>(Nelements, elementList, G2L, wJ, ggeo, gllw, D, \
-                                                                    lambda, q, Aq, skip, Fz);                        \
-    else                                                                                                             \
-      ax_quad_kernel<NQ, NF, AFF, DOT, F><<<grid, block, 0, s>>>(Nelements, elementList, G2L, wJ, ggeo, gllw, D,     \
-                                                                lambda, q, Aq, skip, Fz);                            \
-  } while (0)
-  const bool dot = fuse != nullptr;
-  if (d.Nfields == 1) {
-    if (d.affine) { if (dot) BP_QUAD(1, true, true); else BP_QUAD(1, true, false); }
-    else { if (dot) BP_QUAD(1, false, true); else BP_QUAD(1, false, false); }
-  } else {
-    if (d.affine) { if (dot) BP_QUAD(2, true, true); else BP_QUAD(2, true, false); }
-    else { if (dot) BP_QUAD(2, false, true); else BP_QUAD(2, false, false); }
+  // the line form from about four warps per SM on; below, at the degrees whose
+  // serial line steps show (the two agree within a launch at Nq <= 4), nodes
+  if (NQ > 4 && (int64_t)Nelements * d.Nfields < (int64_t)4 * sm_count() * Sh::SPW) {
+    using Nd = QuadNodeShape<NQ>;
+    const dim3 grid((Nelements + Nd::EPB - 1) / Nd::EPB), block(NQ, NQ, Nd::EPB);
+    if (nblocks) *nblocks = (int)grid.x;
+#define BP_QUAD_NODE(NF)                                                                                             \
+  (d.affine ? (fuse ? ax_quad_node_kernel<NQ, NF, true, true, F> : ax_quad_node_kernel<NQ, NF, true, false, F>)       \
+            : (fuse ? ax_quad_node_kernel<NQ, NF, false, true, F> : ax_quad_node_kernel<NQ, NF, false, false, F>))
+    auto kn = d.Nfields == 1 ? BP_QUAD_NODE(1) : BP_QUAD_NODE(2);
+#undef BP_QUAD_NODE
+    kn<<<grid, block, 0, s>>>(Nelements, elementList, G2L, wJ, ggeo, gllw, D, lambda, q, Aq, skip, Fz);
+    BP_CUDA_TRY(cudaGetLastError());
+    return BP_SUCCESS;
   }
-#undef BP_QUAD
+  const dim3 grid((unsigned)(((int64_t)Nelements * d.Nfields + Sh::EPB - 1) / Sh::EPB));
+  if (nblocks) *nblocks = (int)grid.x;
+  auto k = d.affine ? (fuse ? ax_quad_kernel<NQ, true, true, F> : ax_quad_kernel<NQ, true, false, F>)
+                    : (fuse ? ax_quad_kernel<NQ, false, true, F> : ax_quad_kernel<NQ, false, false, F>);
+  k<<<grid, Sh::THREADS, 0, s>>>(Nelements, d.Nfields, elementList, G2L, wJ, ggeo, gllw, D, lambda, q, Aq, skip, Fz);
   BP_CUDA_TRY(cudaGetLastError());
   return BP_SUCCESS;
 }
