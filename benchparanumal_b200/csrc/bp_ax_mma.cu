@@ -34,18 +34,21 @@
 namespace bp {
 namespace {
 
-template <int NQ>
+template <int NQ, class F = float>
 struct MmaShape {
   static constexpr int S1 = NQ + 4;            // stride of the j index (words of F)
   static constexpr int S2 = NQ * S1 + 4;       // stride of the k index
   static constexpr int ARR = NQ * S2;          // one NQ^3 array, padded
   static constexpr int NP = NQ * NQ * NQ;
   static constexpr int NCOL = NQ * NQ;         // columns of a slab
-  static constexpr int THREADS = 256;
+  // The FP64 arrays leave room for one block per SM; sixteen warps there hide
+  // what eight could not (DMMA pipe 38% busy, 12% occupancy: BK6 p=15 on 14^3
+  // elements 481 -> 396 us with the next field's gather moved ahead, below).
+  // FP32 keeps three blocks of eight.
+  static constexpr int THREADS = sizeof(F) == 8 ? 512 : 256;
   static constexpr int WARPS = THREADS / 32;
   static constexpr int NTILES = NCOL / 8;      // n-tiles of 8 columns
   static constexpr int PER = NP / THREADS;     // nodes per thread in the pointwise phases
-  template <class F>
   static constexpr size_t smem() { return sizeof(F) * 3 * (size_t)ARR; }
   static_assert(NQ % 8 == 0 && NCOL % (8 * WARPS) == 0 && NP % THREADS == 0, "shape");
 };
@@ -131,10 +134,11 @@ struct AFrag<NQ, float> {
 template <int NQ, int TERMS = 1>
 __device__ __forceinline__ void axis_mma(int d, const AFrag<NQ, double>& A, const double* in, double* out, int warp,
                                          int lane) {
-  using Sh = MmaShape<NQ>;
+  using Sh = MmaShape<NQ, double>;
   const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll 1
-  for (int nt = warp; nt < Sh::NTILES; nt += Sh::WARPS) {
+#pragma unroll
+  for (int nt0 = 0; nt0 < Sh::NTILES; nt0 += Sh::WARPS) {   // two tiles at sixteen warps: their chains interleave
+    const int nt = nt0 + warp;
     double c[AFrag<NQ, double>::MT][2];
 #pragma unroll
     for (int mt = 0; mt < AFrag<NQ, double>::MT; ++mt) c[mt][0] = c[mt][1] = 0.0;
@@ -198,13 +202,13 @@ __device__ __forceinline__ void axis_mma(int d, const AFrag<NQ, float>& A, const
 }
 
 template <int NQ, int NF, bool DOT, class F, int TERMS = 3>
-__global__ void __launch_bounds__(MmaShape<NQ>::THREADS, sizeof(F) == 4 ? 2 : 1)
+__global__ void __launch_bounds__((MmaShape<NQ, F>::THREADS), sizeof(F) == 4 ? 2 : 1)
 ax_mma_affine_kernel(int Nelements, const int32_t* __restrict__ elementList, const int32_t* __restrict__ G2L,
                      const F* __restrict__ wJ, const F* __restrict__ ggeo, const F* __restrict__ gllw,
                      const F* __restrict__ Dg, F lambda, const F* __restrict__ q, F* __restrict__ Aq,
                      const int* __restrict__ skip, CgFuse fuse) {
   if (skip && *skip) return;
-  using Sh = MmaShape<NQ>;
+  using Sh = MmaShape<NQ, F>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   F* sA = reinterpret_cast<F*>(smem_raw);   // q, then the r gradient, flux and divergence
   F* sU1 = sA + Sh::ARR;                    // the s gradient, flux and divergence
@@ -225,7 +229,21 @@ ax_mma_affine_kernel(int Nelements, const int32_t* __restrict__ elementList, con
   Dgrad.template load<false>(sD, lane);
   Ddiv.template load<true>(sD, lane);
 
+  // The next field's q is gathered while this one computes: its indices are
+  // asked for before the gradients, its values after them.
   double pdot = 0.0;
+  F rn[Sh::PER];
+  int32_t idn[Sh::PER];
+  auto load_ids = [&](int f) {
+#pragma unroll
+    for (int c = 0; c < Sh::PER; ++c) idn[c] = __ldg(G2L + ((size_t)e * NF + f) * Sh::NP + t + c * Sh::THREADS);
+  };
+  auto load_q = [&]() {
+#pragma unroll
+    for (int c = 0; c < Sh::PER; ++c) rn[c] = idn[c] >= 0 ? __ldg(q + idn[c]) : F(0);
+  };
+  load_ids(0);
+  load_q();
 #pragma unroll 1
   for (int f = 0; f < NF; ++f) {
     const size_t lbase = ((size_t)e * NF + f) * Sh::NP;
@@ -233,17 +251,18 @@ ax_mma_affine_kernel(int Nelements, const int32_t* __restrict__ elementList, con
 #pragma unroll
     for (int c = 0; c < Sh::PER; ++c) {
       const int n = t + c * Sh::THREADS;
-      const int id = __ldg(G2L + lbase + n);
-      rq[c] = id >= 0 ? q[id] : F(0);
+      rq[c] = rn[c];
       const int i = n % NQ, j = (n / NQ) % NQ, k = n / (NQ * NQ);
       sA[k * Sh::S2 + j * Sh::S1 + i] = rq[c];
     }
+    if (f + 1 < NF) load_ids(f + 1);
     __syncthreads();
     // gradients: s and t from q, then r over q itself
     axis_mma<NQ, TERMS>(1, Dgrad, sA, sU1, warp, lane);
     axis_mma<NQ, TERMS>(2, Dgrad, sA, sU2, warp, lane);
     __syncthreads();
     axis_mma<NQ, TERMS>(0, Dgrad, sA, sA, warp, lane);
+    if (f + 1 < NF) load_q();
     __syncthreads();
     // fluxes w G (ur, us, ut), node by node
 #pragma unroll
@@ -441,8 +460,8 @@ template <int NQ, class F>
 int launch_mma_nq(const bp_ax_desc_t& d, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                   const F* wJ, const F* ggeo, const F* gllw, const F* D, F lambda, const F* q, F* Aq,
                   const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks) {
-  using Sh = MmaShape<NQ>;
-  const size_t smem = Sh::template smem<F>();
+  using Sh = MmaShape<NQ, F>;
+  const size_t smem = Sh::smem();
   const CgFuse Fz = fuse ? *fuse : CgFuse{};
   if (nblocks) *nblocks = Nelements;
   // BP_MMA_TF32_TERMS=1 (FP32 only): plain TF32 products instead of the split
