@@ -2,7 +2,8 @@
 // solves (reference: BP/BP5/src/bp5{Setup,Operator,Run}.cpp,
 // libs/core/linearSolverCG.cpp:62-156).
 //
-// CG runs with every scalar on the device.  One iteration is four kernels:
+// CG runs with every scalar on the device.  One iteration is four kernels
+// (three on small meshes, where the gather forms alpha itself: kFoldParts):
 //   cg_direction_kernel     x += alpha_{k-1} p_{k-1} (deferred),  p = z + beta p
 //   element operator        AqL = A_e p, and block partials of p.Ap = sum_e p_e.(A_e p_e)
 //   cg_alpha_kernel         p.Ap from the partials, alpha = rho / p.Ap
@@ -236,6 +237,63 @@ cg_alpha_kernel(int nparts, const double* __restrict__ parts, CgScalars* sc, dou
   }
 }
 
+// A gather that follows the alpha kernel waits for it to leave the SMs (no
+// programmatic launch): an SM keeps its split between L1 and shared memory
+// while blocks follow one another, and a gather that slips in behind an
+// operator with 224 KB of shared memory per SM is left without the L1 that
+// its indices and shared lines need (packed p=7 22x24x23 to 1e-8: 254 ms
+// against 218; a gather denied its L1 outright 253, denied shared memory 374).
+//
+// Up to this many block partials every block of the gather-update
+// adds them for itself (the same order in each, so the same alpha) and the
+// alpha kernel is left out: a read of at most 8 KB from L2 against a launch
+// with its own grid reduction (FP64, 100 iterations: p=4 16^3 2.75 -> 2.64 ms,
+// p=10 5^3 2.51 -> 1.83 ms; four packed lanes, four sums in each block, lose:
+// p=4 10^3 to 1e-8 6.43 -> 6.69 ms, and keep the kernel).  Beyond, the
+// reads by a thousand blocks cost more than the kernel they save.
+constexpr int kFoldParts = 1024;
+
+// p.Ap of NL lanes from the operator's block partials, in every thread of the
+// block; then alpha of lane l, or its breakdown.  Block 0 records them (the
+// scalars that others read here, rz, rdotr and precon, stay as they are until
+// every block has arrived at the grid sum that ends the kernel).
+template <int NL>
+__device__ __forceinline__ void fold_alpha(int nparts, const double* __restrict__ parts, CgScalars* sc,
+                                           double* hist_alpha, bool (&act)[NL], double (&alpha)[NL]) {
+  __shared__ double s_tmp[NL * (kThreads / 32)];
+  __shared__ double s_pap[NL];
+  double acc[NL];
+#pragma unroll
+  for (int l = 0; l < NL; ++l) acc[l] = 0.0;
+  for (int k = threadIdx.x; k < nparts; k += kThreads)
+#pragma unroll
+    for (int l = 0; l < NL; ++l) acc[l] += __ldg(parts + (size_t)l * nparts + k);
+  block_sum_multi_cg<NL>(acc, s_tmp);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int l = 0; l < NL; ++l) s_pap[l] = acc[l];
+  __syncthreads();
+#pragma unroll
+  for (int l = 0; l < NL; ++l) {
+    if (!act[l]) continue;
+    CgScalars& c = sc[l];
+    const double pAp = s_pap[l], a = (c.precon ? c.rz : c.rdotr) / pAp;
+    const bool bad = !(pAp > 0.0) || !isfinite(a);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      c.pAp = pAp;
+      if (bad) {
+        c.breakdown = 1;
+        c.done = 1;
+      } else {
+        c.alpha = a;
+        if (hist_alpha) hist_alpha[c.iter] = a;
+      }
+    }
+    act[l] = !bad;
+    alpha[l] = a;
+  }
+}
+
 // blocks of cg_alpha_kernel: about four partials per thread
 static int alpha_grid(int nparts) {
   int g = (nparts + 4 * kThreads - 1) / (4 * kThreads);
@@ -254,15 +312,28 @@ static int alpha_grid(int nparts) {
 // also asks the host for a reliable update.
 template <class V>
 constexpr int kGatherRows = sizeof(V) == 4 ? 4 : 1;
-template <class V, int RU>
+template <class V, int RU, bool FOLD>
 __global__ void __launch_bounds__(kThreads)
 cg_gather_update_kernel(int32_t Nrows, const int32_t* __restrict__ rowStarts, const int32_t* __restrict__ colIds,
                         const V* __restrict__ AqL, V* __restrict__ r, const V* __restrict__ invD, CgScalars* sc,
-                        double* hist_rnorm, double* partials, unsigned int* counter) {
+                        double* hist_rnorm, double* partials, unsigned int* counter, int nparts,
+                        const double* __restrict__ parts, double* hist_alpha) {
   pdl_wait();
   pdl_release();
-  if (sc->done) return;
-  const V alpha = (V)sc->alpha;
+  V alpha;
+  if (FOLD) {
+    // done may be set by block 0 while others start (a breakdown): they reach
+    // the same verdict, so whichever way a block leaves, all leave
+    if (*(volatile int*)&sc->done) return;
+    bool act[1] = {true};
+    double a[1];
+    fold_alpha<1>(nparts, parts, sc, hist_alpha, act, a);
+    if (!act[0]) return;
+    alpha = (V)a[0];
+  } else {
+    if (sc->done) return;
+    alpha = (V)sc->alpha;
+  }
   const bool precon = sc->precon != 0;
   const int32_t stride = kThreads * gridDim.x;
   double acc[2] = {0.0, 0.0};
@@ -611,6 +682,8 @@ struct bp_solver_s {
   DeviceArray<CgScalars> sc;
   CgScalars* scal = nullptr;   // the CG scalars: sc.ptr, or a slot of a batch's array
   int64_t launches = 0;        // kernels launched (graph nodes included) since the solve began
+  int kernels_per_it = 4;      // kernels of the iteration enqueued last
+  int graph_kernels = 0, graph32_kernels = 0;   // kernels of the captured graphs
   int hist_len = 0;
   // graph of kChunk iterations, keyed by the vectors it was captured for
   cudaGraphExec_t graph = nullptr;
@@ -787,10 +860,14 @@ static int enqueue_iteration(bp_solver_s* S, V* x, V* r, V* p, V* p_alt, V* AqL,
     fuse.partials = S->fuse_partials.ptr;
     BP_TRY(elem_apply<V>(S, o, p, AqL, &S->scal->done, s, &fuse, &nparts));
   }
-  BP_CUDA_TRY(launch_pdl(cg_alpha_kernel<1>, alpha_grid(nparts), kThreads, 0, s, nparts, S->fuse_partials.ptr,
-                         S->scal, hist_alpha, S->partials.ptr, S->counter.ptr));
-  BP_CUDA_TRY(launch_pdl(cg_gather_update_kernel<V, kGatherRows<V>>, g, kThreads, 0, s, N, m->rowStarts.ptr,
-                         m->colIds.ptr, AqL, r, invD, S->scal, hist_rnorm, S->partials.ptr, S->counter.ptr));
+  const bool fold = nparts <= kFoldParts;
+  if (!fold)
+    BP_CUDA_TRY(launch_pdl(cg_alpha_kernel<1>, alpha_grid(nparts), kThreads, 0, s, nparts, S->fuse_partials.ptr,
+                           S->scal, hist_alpha, S->partials.ptr, S->counter.ptr));
+  auto gather = fold ? cg_gather_update_kernel<V, kGatherRows<V>, true> : cg_gather_update_kernel<V, kGatherRows<V>, false>;
+  BP_CUDA_TRY(launch_kernel(fold, gather, g, kThreads, 0, s, N, m->rowStarts.ptr, m->colIds.ptr, AqL, r, invD, S->scal,
+                         hist_rnorm, S->partials.ptr, S->counter.ptr, nparts, S->fuse_partials.ptr, hist_alpha));
+  S->kernels_per_it = 2 + (dir ? 0 : 1) + (fold ? 0 : 1);
   return BP_SUCCESS;
 }
 
@@ -853,6 +930,7 @@ static int ensure_graph(bp_solver_s* S, double* x, double* r, cudaStream_t s) {
   if (S->graph && S->g_x == x && S->g_r == r) return BP_SUCCESS;
   BP_TRY(prepare64(S, s));
   BP_TRY(capture(&S->graph, s, body64, S, x, r));
+  S->graph_kernels = S->kernels_per_it * kChunk;
   S->g_x = x;
   S->g_r = r;
   return BP_SUCCESS;
@@ -923,7 +1001,7 @@ static int solve_fp64(bp_solver_s* S, double* x, double* r, double tol, int maxi
   CgScalars h{};
   for (int c = 0; c < nchunks; ++c) {
     BP_CUDA_TRY(cudaGraphLaunch(S->graph, s));
-    S->launches += (S->dir64 ? 3 : 4) * kChunk;
+    S->launches += S->graph_kernels;
     if (tol > 0.0 && c + 1 < nchunks) {
       BP_TRY(read_scalars(S, h, s));
       if (h.done) break;
@@ -977,6 +1055,7 @@ static int solve_mixed(bp_solver_s* S, double* x, double* r, double tol, int max
   if (!S->graph32) {
     BP_TRY(prepare32(S, s));
     BP_TRY(capture(&S->graph32, s, body32, S, nullptr, nullptr));
+    S->graph32_kernels = S->kernels_per_it * kChunk;
   }
   S->launches = 0;
   if (record_events) BP_CUDA_TRY(cudaEventRecord(S->ev0, s));
@@ -990,7 +1069,7 @@ static int solve_mixed(bp_solver_s* S, double* x, double* r, double tol, int max
       ++updates;
     } else {
       BP_CUDA_TRY(cudaGraphLaunch(S->graph32, s));
-      S->launches += (S->dir32 ? 3 : 4) * kChunk;
+      S->launches += S->graph32_kernels;
     }
     BP_TRY(read_scalars(S, h, s));
     if (h.breakdown) break;
@@ -1254,6 +1333,7 @@ struct BatchUnit {
   int sys = -1;                  // the standalone system (G == nullptr)
   int slot0 = 0, lanes = 1;      // its CG scalar slots
   double weight = 0.0;           // lane-nodes of element data per iteration
+  int kernels = 0;                              // kernels of the graph
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t posted = nullptr;  // the host copy of its scalars has landed
   int stream = -1;               // stream of the pool while in flight
@@ -1338,9 +1418,10 @@ static int grp_iteration(CgGroup* G, cudaStream_t s) {
   BP_CUDA_TRY(launch_pdl(cg_alpha_kernel<PK>, alpha_grid(nparts), kThreads, 0, s, nparts, G->parts.ptr, G->sc,
                          nullptr, G->gparts.ptr, G->gcount.ptr));
   const int gg = vec_grid_wave(reinterpret_cast<const void*>(&grp_gather_update_kernel<PK>), N);
-  BP_CUDA_TRY(launch_pdl(grp_gather_update_kernel<PK>, gg, kThreads, 0, s, N, m->rowStarts.ptr, m->colIds.ptr,
-                         reinterpret_cast<const T*>(G->AqL32.ptr), reinterpret_cast<T*>(G->r32.ptr), S->invD32.ptr,
-                         G->sc, G->gparts.ptr, G->gcount.ptr));
+  BP_CUDA_TRY(launch_kernel(false, grp_gather_update_kernel<PK>, gg, kThreads, 0, s, N, m->rowStarts.ptr,
+                            m->colIds.ptr, reinterpret_cast<const T*>(G->AqL32.ptr),
+                            reinterpret_cast<T*>(G->r32.ptr), S->invD32.ptr, G->sc, G->gparts.ptr, G->gcount.ptr));
+  S->kernels_per_it = G->dir ? 3 : 4;
   return BP_SUCCESS;
 }
 
@@ -1507,6 +1588,7 @@ static int unit_capture(bp_batch_s* B, BatchUnit& u, cudaStream_t s) {
   ce = cudaGraphInstantiate(&u.graph, g, 0);
   cudaGraphDestroy(g);
   BP_CUDA_TRY(ce);
+  u.kernels = (u.G && u.G->persist ? 1 : (u.G ? u.G->base : B->sys_solver[u.sys])->kernels_per_it) * kBatchChunk;
   return BP_SUCCESS;
 }
 
@@ -1617,8 +1699,7 @@ static int batch_solve(bp_batch_s* B, double tol, int maxit, bp_solve_stats_t* s
       if (running) {
         BP_CUDA_TRY(cudaGraphLaunch(u.graph, st));
         bp_solver_s* us = u.G ? u.G->base : B->sys_solver[u.sys];
-        const bool ud = u.G ? u.G->dir : (B->mixed ? us->dir32 : us->dir64);
-        us->launches += ((u.G && u.G->persist) ? 1 : ud ? 3 : 4) * kBatchChunk;
+        us->launches += u.kernels;
         BP_TRY(unit_post(B, u, st));
         ++a;
         continue;
