@@ -253,45 +253,17 @@ cg_alpha_kernel(int nparts, const double* __restrict__ parts, CgScalars* sc, dou
 // reads by a thousand blocks cost more than the kernel they save.
 constexpr int kFoldParts = 1024;
 
-// p.Ap of NL lanes from the operator's block partials, in every thread of the
-// block; then alpha of lane l, or its breakdown.  Block 0 records them (the
-// scalars that others read here, rz, rdotr and precon, stay as they are until
-// every block has arrived at the grid sum that ends the kernel).
-template <int NL>
-__device__ __forceinline__ void fold_alpha(int nparts, const double* __restrict__ parts, CgScalars* sc,
-                                           double* hist_alpha, bool (&act)[NL], double (&alpha)[NL]) {
-  __shared__ double s_tmp[NL * (kThreads / 32)];
-  __shared__ double s_pap[NL];
-  double acc[NL];
-#pragma unroll
-  for (int l = 0; l < NL; ++l) acc[l] = 0.0;
-  for (int k = threadIdx.x; k < nparts; k += kThreads)
-#pragma unroll
-    for (int l = 0; l < NL; ++l) acc[l] += __ldg(parts + (size_t)l * nparts + k);
-  block_sum_multi_cg<NL>(acc, s_tmp);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int l = 0; l < NL; ++l) s_pap[l] = acc[l];
+// p.Ap from the operator's block partials, the same bits in every thread of
+// every block (each block adds all of them in the same order).
+__device__ __forceinline__ double fold_pap(int nparts, const double* __restrict__ parts) {
+  __shared__ double s_tmp[kThreads / 32];
+  __shared__ double s_pap;
+  double acc = 0.0;
+  for (int k = threadIdx.x; k < nparts; k += kThreads) acc += __ldg(parts + k);
+  acc = block_sum_cg(acc, s_tmp);
+  if (threadIdx.x == 0) s_pap = acc;
   __syncthreads();
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    if (!act[l]) continue;
-    CgScalars& c = sc[l];
-    const double pAp = s_pap[l], a = (c.precon ? c.rz : c.rdotr) / pAp;
-    const bool bad = !(pAp > 0.0) || !isfinite(a);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      c.pAp = pAp;
-      if (bad) {
-        c.breakdown = 1;
-        c.done = 1;
-      } else {
-        c.alpha = a;
-        if (hist_alpha) hist_alpha[c.iter] = a;
-      }
-    }
-    act[l] = !bad;
-    alpha[l] = a;
-  }
+  return s_pap;
 }
 
 // blocks of cg_alpha_kernel: about four partials per thread
@@ -320,24 +292,32 @@ cg_gather_update_kernel(int32_t Nrows, const int32_t* __restrict__ rowStarts, co
                         const double* __restrict__ parts, double* hist_alpha) {
   pdl_wait();
   pdl_release();
+  // One rule for every scalar of sc that a block reads here, done among them:
+  // it changes in the last block to arrive at the grid sum below, when all
+  // threads of all blocks have read it.  So a breakdown found by the fold is
+  // not recorded on the spot: its blocks leave their rows alone, arrive like
+  // any others (the counter ends at zero), and the last one records it.
+  if (sc->done) return;
+  bool bad = false;
   V alpha;
   if (FOLD) {
-    // done may be set by block 0 while others start (a breakdown): they reach
-    // the same verdict, so whichever way a block leaves, all leave
-    if (*(volatile int*)&sc->done) return;
-    bool act[1] = {true};
-    double a[1];
-    fold_alpha<1>(nparts, parts, sc, hist_alpha, act, a);
-    if (!act[0]) return;
-    alpha = (V)a[0];
+    const double pAp = fold_pap(nparts, parts), a = (sc->precon ? sc->rz : sc->rdotr) / pAp;
+    bad = !(pAp > 0.0) || !isfinite(a);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // read by no block of this launch
+      sc->pAp = pAp;
+      if (!bad) {
+        sc->alpha = a;
+        if (hist_alpha) hist_alpha[sc->iter] = a;
+      }
+    }
+    alpha = (V)a;
   } else {
-    if (sc->done) return;
     alpha = (V)sc->alpha;
   }
   const bool precon = sc->precon != 0;
   const int32_t stride = kThreads * gridDim.x;
   double acc[2] = {0.0, 0.0};
-  for (int32_t row0 = blockIdx.x * kThreads + threadIdx.x; row0 < Nrows; row0 += RU * stride) {
+  for (int32_t row0 = blockIdx.x * kThreads + threadIdx.x; row0 < (bad ? 0 : Nrows); row0 += RU * stride) {
     V rold[RU], dinv[RU], s[RU];
     int32_t c[RU], e[RU];
 #pragma unroll
@@ -373,6 +353,11 @@ cg_gather_update_kernel(int32_t Nrows, const int32_t* __restrict__ rowStarts, co
   }
   double tot[2];
   if (grid_sum_cg<2>(acc, partials, counter, tot) && threadIdx.x == 0) {
+    if (bad) {
+      sc->breakdown = 1;
+      sc->done = 1;
+      return;
+    }
     sc->rdotr_prev = sc->rdotr;
     sc->rdotr = tot[0];
     if (precon) {

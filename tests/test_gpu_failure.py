@@ -76,3 +76,37 @@ def test_batch_reports_numeric_error_of_one_system(gpu):
     with pytest.raises(gpu.BPError, match="breakdown") as e:
         B.solve(tol=1e-8, maxit=300)
     assert e.value.code == gpu.BP_ERROR_NUMERIC
+
+
+# An indefinite operator (lambda below minus the Rayleigh quotient of the gathered
+# analytic forcing, 783 and 164 on these meshes): p.Ap < 0 in the first iteration
+# of the one right-hand side, positive in the first ones of the random one.  11^3 nodes on 10^3 elements:
+# at most 1000 block partials, so the gather forms alpha itself, in a grid of more
+# blocks than rest on the chip beside one another; 6^3 p=4: one wave.
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+@pytest.mark.parametrize("N,n,lam", [(10, 10, -1000.0), (4, 6, -200.0)])
+def test_breakdown_in_the_gather_leaves_the_solver_usable(gpu, N, n, lam, precision):
+    gm = gpu.Mesh(n, n, n, N=N, pert=0.1)
+    tol = 1e-30 if precision == "MIXED" else 0.0
+
+    def good(S):
+        x, r = gpu.DeviceBuffer.from_host(np.zeros(gm.Ngather)), S.rhs("RANDOM", 3)
+        st, hist, alpha = S.solve(x, r, tol=tol, maxit=3)
+        return st, hist, alpha, x.download(), r.download()
+
+    want = good(gpu.BP(gm, lam=lam, precision=precision))
+    assert want[0].iterations == 3
+    if precision == "FP64":   # operator, gather and init, one chunk of 20 iterations of three kernels, last x update
+        assert want[0].kernel_launches == 3 + 20 * 3 + 1
+    S = gpu.BP(gm, lam=lam, precision=precision)
+    b = S.rhs("ANALYTIC").download()
+    for _ in range(10):
+        x, r = gpu.DeviceBuffer.from_host(np.zeros(gm.Ngather)), gpu.DeviceBuffer.from_host(b)
+        with pytest.raises(gpu.BPError, match="breakdown") as e:
+            S.solve(x, r, tol=tol, maxit=20)
+        assert e.value.code == gpu.BP_ERROR_NUMERIC
+        assert np.array_equal(r.download(), b)      # no row was updated with the rejected alpha
+        assert not np.any(x.download())
+        got = good(S)
+        for a, w in zip(got[1:], want[1:]):
+            assert np.array_equal(a, w)
