@@ -282,7 +282,12 @@ static int launch_ax_nq(const bp_ax_desc_t& d, int32_t Nelements, const int32_t*
   };
   int form = forms[0];
   const int v = ax_variant();
-  if (v != AX_AUTO) {
+  if (!d.affine && reinterpret_cast<uintptr_t>(ggeo) % (2 * sizeof(F))) {
+    // stored factors not aligned to two elements: the pencil kernel alone reads
+    // them one by one, whatever form is forced or recorded for aligned ones (and
+    // nothing is recorded from here)
+    form = FORM_PENCIL;
+  } else if (v != AX_AUTO) {
     form = v == AX_MMA ? FORM_MMA : v == AX_TMA ? FORM_TMA : v == AX_LINE ? FORM_LINE : FORM_PENCIL;
   } else {
     const TuneConfig cfg{0, NQ, d.Nfields, d.affine, (int)sizeof(F), 1, fuse != nullptr, element_class(Nelements)};

@@ -32,6 +32,34 @@ def test_hex_permuted_subset(gpu, oracle, monkeypatch, N, affine, nf):
     assert _rel(got[els], want[els]) < 1e-12
 
 
+# Stored factors aligned to one element only are read one by one by the pencil
+# form, whatever form is forced or recorded for aligned calls, and record nothing.
+@pytest.mark.parametrize("variant", ["", "line"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("N,nf", [(4, 1), (7, 1), (7, 3)])
+def test_factors_aligned_to_one_element(gpu, oracle, monkeypatch, N, nf, dtype, variant):
+    if variant:
+        monkeypatch.setenv("BP_AX_VARIANT", variant)
+    om, gm = oracle.Mesh(3, 2, 2, N, Nfields=nf, pert=0.1), gpu.Mesh(3, 2, 2, N=N, Nfields=nf, pert=0.1)
+    d, v = gpu.AxDesc(5 if nf == 1 else 6, N, 0, nf), gm.view
+    q = (2 * oracle.random(5, om.Ngather) - 1).astype(dtype)
+    ops = {k: gpu.DeviceBuffer.from_host(gm.array(k).astype(dtype)) for k in ("wJ", "gllw", "D")}
+    g = gm.array("ggeo").astype(dtype)
+    bufs = [gpu.DeviceBuffer.from_host(np.concatenate([np.zeros(off, dtype), g])) for off in (0, 1)]
+    dq, f = gpu.DeviceBuffer.from_host(q), gpu.lib().bp_ax_hex3d if dtype == np.float64 else gpu.lib().bp_ax_hex3d_f32
+    out, forms = [], []
+    for off, b in enumerate(bufs):
+        dA = gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan, dtype))
+        gpu._check(f(gpu.ctypes.byref(d), gm.E, v.elementList, v.GlobalToLocal, ops["wJ"].ptr,
+                     b.ptr + off * g.itemsize, ops["gllw"].ptr, ops["D"].ptr, 1.0, dq.ptr, dA.ptr, None))
+        out.append(dA.download().astype(np.float64))
+        forms.append(gpu.tune_report(0, N, nf, 0, g.itemsize, 1, 0, gm.E)[0])
+    want = om.ax(q.astype(np.float64))
+    for o in out:
+        assert _rel(o, want) < (1e-12 if dtype == np.float64 else 2e-5)
+    assert forms[0] == forms[1]
+
+
 @pytest.mark.parametrize("N", [1, 2, 3, 4, 5, 6, 7, 8, 10])
 def test_packed_lines(gpu, oracle, monkeypatch, N):
     monkeypatch.setenv("BP_AX_VARIANT", "line")
