@@ -75,9 +75,9 @@ ax_quad_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementLi
   const int lane = threadIdx.x & 31, sl = lane / NQ;
   const bool on = sl < SPW;                               // the last lanes own no line
   const int slot = (threadIdx.x >> 5) * SPW + (on ? sl : 0), x = on ? lane - sl * NQ : 0;
-  const int v = blockIdx.x * Sh::EPB + slot;              // element-major (element, field)
-  const bool valid = on && v < Nelements * Nfields;
-  const int eidx = Nfields == 1 ? v : v / Nfields, f = v - eidx * Nfields;
+  const int64_t v = (int64_t)blockIdx.x * Sh::EPB + slot;  // element-major (element, field); past 2^31 with two fields
+  const bool valid = on && v < (int64_t)Nelements * Nfields;
+  const int eidx = Nfields == 1 ? (int)v : (int)(v / Nfields), f = (int)(v - (int64_t)eidx * Nfields);
   const int e = valid ? elementList[eidx] : 0;
   const size_t lbase = ((size_t)e * Nfields + f) * NP;
   const F* const ge = ggeo + 3 * (size_t)e * (AFFINE ? 1 : NP);

@@ -136,3 +136,26 @@ def test_quad_rejections(gpu):
     with pytest.raises(gpu.BPError):
         gpu.Mesh(3, 3, N=4, Nfields=3, dim=2)
     assert gpu.driver_main("BP3", ["-e", "Quad", "-nx", "4", "-ny", "4"]) != 0
+
+
+def test_more_element_fields_than_31_bits(gpu, oracle):
+    """2^30 + 64 listed elements of two fields: the slot index passes 2^31.  The
+    list repeats the 32 x 32 elements of a small mesh, so that every one of them
+    is listed at its end, too."""
+    gm = gpu.Mesh(32, 32, 1, N=1, Nfields=2, pert=0.1, dim=2)
+    n, E = (1 << 30) + 64, gm.E
+    els = gpu.DeviceBuffer(n, np.int32)
+    first = np.arange(E, dtype=np.int32)[::-1].copy()
+    gpu._check(gpu.lib().bp_memcpy_htod(els.ptr, first.ctypes.data, 4 * E, None))
+    gpu.finish()
+    have = E
+    while have < n:
+        more = min(have, n - have)
+        gpu._check(gpu.lib().bp_memcpy_dtod(els.ptr + 4 * have, els.ptr, 4 * more, None))
+        have += more
+    dq = gpu.DeviceBuffer.from_host(2 * oracle.random(5, gm.Ngather) - 1)
+    want = gpu.DeviceBuffer(gm.NL)
+    gpu.ax_hex3d(gm, dq, want)
+    got = gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
+    gpu.ax_hex3d(gm, dq, got, elementList=els.ptr, Nelements=n)
+    assert np.array_equal(got.download(), want.download())
