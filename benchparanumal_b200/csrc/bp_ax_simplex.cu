@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "bp_cg_device.cuh"
@@ -374,11 +375,22 @@ struct SimplexMmaPlan {
   size_t smem(int Np) const { return sizeof(double) * (size_t)eb() * simplex_kp(Np); }
 };
 
-// The plan with the least estimated time: the rounds of row sets a warp runs,
-// times the tile products, fragment loads and latency of a k step, times the
-// blocks beyond what three per SM hold.  A batch that leaves the chip idle
+// The plan with the least estimated time.  A batch that leaves the chip idle
 // spreads its rows over blockIdx.y, to at most about two blocks per SM.
-static SimplexMmaPlan simplex_mma_plan(int Np, int32_t E, int sms) {
+//
+// A block alone on its SM takes the k steps of its rounds, each with its tile
+// products, fragment loads and a latency, after the gather of its q tile in
+// batches of dependent loads.  The n blocks of the busiest SM follow one
+// another at the pace of the more limiting of their residency (registers or
+// shared memory) and of the SM's DMMA and load pipes.  The weights (in DMMA
+// issue slots) are fitted to 6,500 timings: every plan at 199 problems, triangles
+// p = 3..15 and tetrahedra p = 2..12, 6 to 400,000 elements.  Over these the
+// chosen plan takes 1.024 of the best plan's time on average.  The rule before
+// (rounds times the step, times the waves beyond three blocks per SM) took 1.07
+// and lost to one thread per node at 700-2,100 elements: tetrahedra p=8, 750:
+// 49 us against 44 there and 30 now; p=5, 2,058: 22, 20, 14.
+static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms) {
+  constexpr int regs[5] = {72, 96, 128, 128, 168};   // registers a thread of the kernel takes, by mt
   const int tiles = (Np + 7) / 8;
   SimplexMmaPlan best{1, 1, 1, 1};
   double cost = 1e300;
@@ -391,8 +403,14 @@ static SimplexMmaPlan simplex_mma_plan(int Np, int32_t E, int sms) {
         const int bx = (E + p.eb() - 1) / p.eb();
         p.gy = std::max(1, std::min(sets, 2 * sms / bx));
         const int rounds = (sets + p.gy - 1) / p.gy;
-        const double waves = (double)bx * p.gy / (3 * sms);
-        const double c = std::max(waves, 1.0) * rounds * (mt * nt + 0.6 * mt + 0.3 * nt + 1.5);
+        const double n = (bx * (int64_t)p.gy + sms - 1) / sms;
+        const double steps = (double)rounds * C * ((Np + 3) / 4);
+        const double gathers = p.eb() * ((Np + 3) / 4 * 4) / (6.0 * 32 * kMmaWarps);
+        const int resident = (int)std::min<size_t>(65536 / (regs[mt - 1] * 32 * kMmaWarps),
+                                                   227 * 1024 / (p.smem(Np) + 1024));
+        const double alone = steps * (mt * nt + 0.7 * mt + 3.4 * nt + 7) + 60 * std::ceil(gathers);
+        const double pipes = steps * (0.8 * mt * nt + 0.4 * mt) + 11 * gathers;
+        const double c = alone + (n - 1) * std::max(alone / resident, pipes);
         if (c < cost) {
           cost = c;
           best = p;
@@ -422,7 +440,7 @@ static int launch_ax_simplex_mma(int N, int32_t E, const int32_t* elementList, c
                                  const double* q, double* Aq, const int* skip, cudaStream_t s, double* partials,
                                  int* nblocks) {
   const int Np = simplex_np(C == 4 ? 2 : 3, N);
-  const SimplexMmaPlan p = simplex_mma_plan(Np, E, sm_count());
+  const SimplexMmaPlan p = simplex_mma_plan(C, Np, E, sm_count());
 #define BP_SIMPLEX_MMA(MT, NT)                                                                                     \
   if (p.mt == MT && p.nt == NT)                                                                                    \
     return launch_simplex_mma<C, MT, NT>(p, Np, E, elementList, G2L, wJ, ggeo, S, MM, lambda, q, Aq, skip, s, partials, \
