@@ -49,7 +49,7 @@ EXPORTS = [
     "bp_solver_create", "bp_solver_destroy", "bp_solver_size", "bp_solver_operator", "bp_solver_rhs",
     "bp_solver_diagonal", "bp_solver_solve", "bp_solver_solve_host", "bp_driver_main",
     "bp_box_numbering", "bp_basis_gll", "bp_box_vertices", "bp_operator_hex3d_noalloc", "bp_ogs_check",
-    "bp_test_wait_timeout", "bp_tune_report", "bp_tune_reset",
+    "bp_test_wait_timeout", "bp_test_operator_plan", "bp_tune_report", "bp_tune_reset",
     "bp_ax_cub_hex3d", "bp_mesh_cubature", "bp_mesh_cubature_view", "bp_basis_cubature", "bp_basis_tri2d", "bp_basis_tet3d",
     "bp_batch_create", "bp_batch_destroy", "bp_batch_systems", "bp_batch_system_info", "bp_batch_solve",
     "bp_batch_vectors", "bp_batch_solver", "bp_ax_hex3d_f32", "bp_convert_f64_f32", "bp_ax_hex3d_f32_multi",
@@ -177,6 +177,7 @@ def lib():
             "bp_box_vertices": [ctypes.POINTER(BoxDesc), vp, vp, vp],
             "bp_ogs_check": [ctypes.c_int64, vp, i32, vp, vp],
             "bp_test_wait_timeout": [ctypes.c_int],
+            "bp_test_operator_plan": [ctypes.c_int] * 5 + [i32, vp],
             "bp_tune_report": [i32] * 8 + [ctypes.POINTER(i32), ctypes.POINTER(i32), vp, vp, i32],
             "bp_tune_reset": [],
             "bp_operator_hex3d_noalloc": [ctypes.POINTER(AxDesc), i32, vp, vp, vp, vp, vp, vp, dbl, i32, i32, vp,

@@ -15,6 +15,19 @@
 #include "bp_internal.hpp"
 
 namespace bp {
+
+// The line form from the warps per SM on at which it overtakes the node form,
+// measured at 1 to 40 warps per SM, all degrees, both precisions and field
+// counts: with stored factors between 4 (p=12) and 11 (FP32 p=2), at most
+// degrees near 8 (node/line time at p=5 FP64 0.88 at 6 warps, 1.02 at 8, 1.13
+// at 16; p=8 FP32 0.83, 0.97, 1.39); affine, where the line form's loads are
+// fewer, between 2 and 5 (p=5 FP64 0.78 at 2, 0.93 at 3, 1.03 at 6).  Two
+// fields, whose factors the node form reads once, somewhat later.
+bool quad_line_form(int N, int affine, int Nfields, int32_t Nelements) {
+  const int warps = affine ? 2 + Nfields : 6 + 2 * Nfields;
+  return (int64_t)Nelements * Nfields >= (int64_t)warps * sm_count() * (32 / (N + 1));
+}
+
 namespace {
 
 // One warp serves SPW element(-field)s of NQ lines each; a thread owns column x
@@ -77,7 +90,7 @@ ax_quad_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementLi
   const int slot = (threadIdx.x >> 5) * SPW + (on ? sl : 0), x = on ? lane - sl * NQ : 0;
   const int64_t v = (int64_t)blockIdx.x * Sh::EPB + slot;  // element-major (element, field); past 2^31 with two fields
   const bool valid = on && v < (int64_t)Nelements * Nfields;
-  const int eidx = Nfields == 1 ? (int)v : (int)(v / Nfields), f = (int)(v - (int64_t)eidx * Nfields);
+  const int eidx = (int)(v >> (Nfields - 1)), f = (int)v & (Nfields - 1);   // one or two fields
   const int e = valid ? elementList[eidx] : 0;
   const size_t lbase = ((size_t)e * Nfields + f) * NP;
   const F* const ge = ggeo + 3 * (size_t)e * (AFFINE ? 1 : NP);
@@ -173,8 +186,8 @@ ax_quad_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementLi
 
 // Node form, for meshes too small to fill the chip with warps: one thread per
 // node, so an element takes Nq dependent steps where the line form takes Nq^2
-// per thread (BK5 p=15, 42 elements: 6.7 us against 12; 100,000 elements 39
-// against 60 us the other way).
+// per thread (BK5 p=15, 42 elements: 6.7 us against 12; 100,000 elements 60
+// against 39 us the other way).
 template <int NQ>
 struct QuadNodeShape {
   static constexpr int EPB0 = 256 / (NQ * NQ);
@@ -261,9 +274,7 @@ static int launch_quad_nq(const bp_ax_desc_t& d, int32_t Nelements, const int32_
                           const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks) {
   using Sh = QuadShape<NQ>;
   const CgFuse Fz = fuse ? *fuse : CgFuse{};
-  // the line form from about four warps per SM on; below, at the degrees whose
-  // serial line steps show (the two agree within a launch at Nq <= 4), nodes
-  if (NQ > 4 && (int64_t)Nelements * d.Nfields < (int64_t)4 * sm_count() * Sh::SPW) {
+  if (!quad_line_form(d.N, d.affine, d.Nfields, Nelements)) {
     using Nd = QuadNodeShape<NQ>;
     const dim3 grid((Nelements + Nd::EPB - 1) / Nd::EPB), block(NQ, NQ, Nd::EPB);
     if (nblocks) *nblocks = (int)grid.x;

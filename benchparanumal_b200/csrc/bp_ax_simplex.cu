@@ -492,6 +492,16 @@ static int launch_ax_simplex_any(int dim, int N, int32_t Nelements, const int32_
                                    nblocks);
 }
 
+void simplex_plan(int dim, int N, int32_t Nelements, int32_t* plan) {
+  const int Np = simplex_np(dim, N);
+  const SimplexMmaPlan p =
+      Np < 8 ? SimplexMmaPlan{0, 0, 0, 0} : simplex_mma_plan(dim == 2 ? 4 : 7, Np, Nelements, sm_count());
+  plan[0] = p.mt;
+  plan[1] = p.nt;
+  plan[2] = p.wm;
+  plan[3] = p.gy;
+}
+
 int launch_ax_simplex(int dim, int N, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                       const double* wJ, const double* ggeo, const double* S, const double* MM, double lambda,
                       const double* q, double* Aq, const int* skip, cudaStream_t s, double* partials, int* nblocks) {

@@ -279,6 +279,7 @@ struct bp_solver_s;
 
 // ---- simplex elements: Tri2D (dim 2), Tet3D (dim 3) (bp_ax_simplex.cu) ----
 namespace bp {
+void simplex_plan(int dim, int N, int32_t Nelements, int32_t* plan);
 int launch_ax_simplex(int dim, int N, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                       const double* wJ, const double* ggeo, const double* S, const double* MM, double lambda,
                       const double* q, double* Aq, const int* skip, cudaStream_t s, double* partials = nullptr,
@@ -450,6 +451,7 @@ int launch_ax_mma_packed(int pk, const bp_ax_desc_t& d, int32_t Nelements, const
 // Quad2D forms (bp_ax_quad.cu): the BP5/BP6 element operator (FP64 and FP32;
 // 1 with a fused direction update, which it does not take), the forcing, the
 // lumped mass and the element diagonal
+bool quad_line_form(int N, int affine, int Nfields, int32_t Nelements);   // rather than the node form
 int launch_ax_quad(const bp_ax_desc_t& d, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                    const double* wJ, const double* ggeo, const double* gllw, const double* D, double lambda,
                    const double* q, double* Aq, const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks);

@@ -546,6 +546,13 @@ int bp_ogs_check(int64_t Nlocal, const int32_t* GlobalToLocal, int32_t Ngather, 
    usable), BP_SUCCESS otherwise.  Allocates its own small buffers. */
 int bp_test_wait_timeout(int withhold_slice);
 
+/* Test hook: how the Quad2D (dim 2) or the FP64 simplex operator (simplex != 0)
+   would run on this many elements on the current device.  Quad2D: plan[0] = 1
+   for the line form, 0 for the node form.  Simplex: 8-node tiles and 8-element
+   tiles per warp, warps along the nodes, blocks along the nodes (all 0 below 8
+   nodes per element, where a thread serves a node). */
+int bp_test_operator_plan(int dim, int simplex, int N, int affine, int Nfields, int32_t Nelements, int32_t* plan);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,10 +1,10 @@
-"""The line forms of the BP5/BP6 operators where a block or warp serves several
-(element, field) slots: permuted partial element lists on Hex3D (one value per
-node and four packed), Quad2D on both sides of the rule that picks its form,
-and the simplex operator's row split, against the FP64 oracle.
+"""The line forms of the BP5/BP6 operators on Hex3D where a block serves several
+(element, field) slots: permuted partial element lists (one value per node) and
+four packed right-hand sides, against the FP64 oracle; and stored factors of any
+alignment.
 
-1e-12 relative in FP64 as elsewhere (sums of at most 136 terms on the simplex,
-16 per 1D step); 2e-5 in FP32, the bar of the other FP32 operators."""
+1e-12 relative in FP64 as elsewhere (sums of at most 16 terms per 1D step);
+2e-5 in FP32, the bar of the other FP32 operators."""
 import numpy as np
 import pytest
 
@@ -76,30 +76,3 @@ def test_packed_lines(gpu, oracle, monkeypatch, N):
     got = dA.download().reshape(-1, 4).astype(np.float64)
     for k in range(4):
         assert _rel(got[:, k], om.ax(q[:, k].astype(np.float64))) < 2e-5
-
-
-# 3 x 2 elements: the node form above Nq = 4; 40 x 31: the line form up to Nq = 16.
-# Against numpy on the mesh's own factors: the oracle's factors differ from the
-# library's by the cancellation in the coordinate derivatives (1.6e-12 of the
-# result at N = 15 on 40 x 31), which is no property of the operator.  Bound:
-# two sums of Nq terms in each direction, 4 Nq 2^-53 < 1e-14 on terms that
-# cancel to a tenth at the most.
-@pytest.mark.parametrize("nx,ny", [(3, 2), (40, 31)])
-@pytest.mark.parametrize("N", [1, 4, 6, 9, 15])
-@pytest.mark.parametrize("affine,nf", [(False, 1), (True, 1), (False, 2), (True, 2)])
-def test_quad_forms(gpu, oracle, nx, ny, N, affine, nf):
-    gm = gpu.Mesh(nx, ny, 1, N=N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1, dim=2)
-    q = 2 * oracle.random(5, gm.Ngather) - 1
-    dq, dA = gpu.DeviceBuffer.from_host(q), gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
-    gpu.ax_hex3d(gm, dq, dA)
-    ids, D, w = gm.array("GlobalToLocal"), gm.array("D").reshape(gm.Nq, gm.Nq), gm.array("gllw")
-    g, J = gm.array("ggeo").reshape(gm.E, -1, 3), gm.array("wJ").reshape(gm.E, -1)
-    if affine:
-        ww = np.outer(w, w).reshape(-1)
-        g, J = g * ww[None, :, None], J * ww[None, :]
-    g, J = g.reshape(gm.E, 1, gm.Nq, gm.Nq, 3), J.reshape(gm.E, 1, gm.Nq, gm.Nq)
-    u = np.where(ids >= 0, q[np.maximum(ids, 0)], 0.0).reshape(gm.E, nf, gm.Nq, gm.Nq)
-    ur, us = u @ D.T, np.einsum("jm,efmi->efji", D, u)
-    fr, fs = g[..., 0] * ur + g[..., 1] * us, g[..., 1] * ur + g[..., 2] * us
-    want = J * u + fr @ D + np.einsum("mj,efmi->efji", D, fs)
-    assert _rel(dA.download(), want.reshape(-1)) < 1e-13

@@ -98,7 +98,6 @@ def test_quad_cg_history_matches_oracle(gpu, oracle, nx, ny, N, affine, pert, nf
     assert np.all(np.abs(hr - hr_o) <= HIST_TOL * hr_o[0])
 
 
-# affine: the FP32 column form of the operator (one thread per column of nodes)
 @pytest.mark.parametrize("nf,affine", [(1, False), (2, False), (1, True), (2, True)])
 def test_quad_mixed_solve_reaches_tolerance(gpu, oracle, nf, affine):
     pert = 0.0 if affine else 0.1
@@ -158,4 +157,5 @@ def test_more_element_fields_than_31_bits(gpu, oracle):
     gpu.ax_hex3d(gm, dq, want)
     got = gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
     gpu.ax_hex3d(gm, dq, got, elementList=els.ptr, Nelements=n)
-    assert np.array_equal(got.download(), want.download())
+    # the small mesh takes the node form: the same few terms in another order
+    assert _rel(got.download(), want.download()) < 1e-14
