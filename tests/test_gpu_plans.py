@@ -1,6 +1,7 @@
 """Operators whose form or tile plan a rule picks by the number of elements, in
 every form and plan, with the plan asserted: Quad2D on both sides of its rule
-(line and node form, all degrees, FP64 and FP32) and inside CG.
+(line and node form, all degrees, FP64 and FP32) and inside CG; the simplex
+operator's tiles per warp, warps along the nodes and row split.
 
 Against numpy on the mesh's own factors and matrices: an oracle's factors differ
 from the library's by the cancellation in the coordinate derivatives, which is
@@ -99,3 +100,97 @@ def test_quad_line_form_inside_cg(gpu, oracle, N, affine, nf):
     x = gpu.DeviceBuffer.from_host(np.zeros(om.Ngather))
     gpu.BP(gm, precon="JACOBI", precision="MIXED").solve(x, gpu.DeviceBuffer.from_host(b), tol=1e-8, maxit=20000)
     assert np.linalg.norm(b - om.operator(x.download())) <= 1.0001e-8 * np.linalg.norm(b)
+
+
+def _simplex_reference(gm, q):
+    """sum_c f_c(e) X_c q_e over the stiffness matrices and MM (stored node-fastest:
+    row k of an array holds X(:, k))."""
+    C = 3 if gm.dim == 2 else 6
+    S = gm.array("S").reshape(C, gm.Np, gm.Np)
+    g, u = gm.array("ggeo").reshape(gm.E, C), _gathered(gm, q).reshape(gm.E, gm.Np)
+    out = gm.array("wJ").reshape(gm.E, 1) * (u @ gm.array("MM").reshape(gm.Np, gm.Np))
+    for c in range(C):
+        out += g[:, c:c + 1] * (u @ S[c])
+    return out
+
+
+# (dim, degree, cells per direction) and the 8-node tiles, 8-element tiles and warps
+# along the nodes of the plan on 148 SMs.  The permuted list leaves elements out,
+# and the last tile partly empty in the one list or the other.
+PLANS = [(2, 3, 1, 1, 1, 1), (2, 6, 1, 1, 1, 2), (2, 9, 1, 1, 1, 4), (2, 3, 100, 1, 2, 2), (2, 6, 90, 1, 2, 4),
+         (2, 3, 35, 2, 1, 1), (2, 7, 22, 2, 1, 2), (2, 10, 16, 2, 1, 4), (2, 3, 90, 2, 2, 1), (2, 6, 140, 2, 2, 2),
+         (2, 9, 70, 2, 2, 4), (2, 5, 40, 3, 1, 1), (2, 7, 29, 3, 1, 2), (2, 10, 22, 3, 1, 4), (2, 10, 55, 3, 2, 1),
+         (2, 15, 35, 3, 2, 2), (3, 8, 7, 3, 2, 4), (2, 15, 29, 4, 1, 1), (2, 9, 55, 4, 1, 2), (3, 15, 3, 4, 1, 4),
+         (2, 6, 180, 4, 2, 1), (3, 8, 8, 4, 2, 2), (3, 9, 7, 4, 2, 4), (3, 7, 6, 5, 1, 1), (3, 9, 5, 5, 1, 2),
+         (2, 15, 23, 5, 1, 4), (3, 4, 14, 5, 2, 1), (2, 10, 60, 5, 2, 2), (2, 15, 43, 5, 2, 4)]
+
+
+def _simplex_mesh(gpu, dim, N, n):
+    return gpu.Mesh(n, n, n if dim == 3 else 1, N=N, affine=True, dim=dim, simplex=True)
+
+
+def _simplex_apply(gpu, gm, q, els):
+    d, v = gpu.AxDesc(5, gm.N, 1, 1, gm.dim), gm.view
+    f = gpu.lib().bp_ax_tri2d if gm.dim == 2 else gpu.lib().bp_ax_tet3d
+    dq, dA = gpu.DeviceBuffer.from_host(q), gpu.DeviceBuffer.from_host(np.full(gm.NL, np.nan))
+    de = gpu.DeviceBuffer.from_host(els)
+    gpu._check(f(gpu.ctypes.byref(d), els.size, de.ptr, v.GlobalToLocal, v.wJ, v.ggeo, v.S, v.MM, 1.0, dq.ptr, dA.ptr,
+                 None))
+    return dA.download().reshape(gm.E, -1)
+
+
+# A sum over k of Np terms and one over c of at most 7: (Np + 7) 2^-53 of the terms'
+# absolute sum in either order of summation, and that sum beside the result in the
+# maximum norm: both from the same matrices.
+def _simplex_bound(gm, q):
+    C = 3 if gm.dim == 2 else 6
+    u = np.abs(_gathered(gm, q).reshape(gm.E, gm.Np))
+    a = np.abs(gm.array("wJ")).reshape(gm.E, 1) * (u @ np.abs(gm.array("MM").reshape(gm.Np, gm.Np)))
+    for c in range(C):
+        a += np.abs(gm.array("ggeo").reshape(gm.E, C)[:, c:c + 1]) * (u @ np.abs(gm.array("S").reshape(C, gm.Np, gm.Np)[c]))
+    return 2 * (gm.Np + 7) * 2.0 ** -53 * a
+
+
+@pytest.mark.parametrize("dim,N,n,mt,nt,wm", PLANS)
+def test_simplex_plans(gpu, dim, N, n, mt, nt, wm):
+    gm = _simplex_mesh(gpu, dim, N, n)
+    rng = np.random.default_rng(N)
+    q = 2 * rng.random(gm.Ngather) - 1
+    want, bound = _simplex_reference(gm, q), _simplex_bound(gm, q)
+    full, part = np.arange(gm.E, dtype=np.int32), rng.permutation(gm.E)[:gm.E - gm.E // 50 - 1].astype(np.int32)
+    plan = _plan(gpu, dim, True, N, True, 1, gm.E)
+    sms = gpu.ctypes.c_int()
+    gpu._check(gpu.lib().bp_device_info(None, 0, gpu.ctypes.byref(sms)))
+    if sms.value == 148:
+        assert plan[:3] == (mt, nt, wm)
+    for els in (full, part):
+        got = _simplex_apply(gpu, gm, q, els)
+        assert np.all(np.isnan(got[np.setdiff1d(full, els)]))
+        assert np.all(np.abs(got[els] - want[els]) <= bound[els])
+
+
+def test_simplex_plans_cover_every_tile_shape_and_both_row_splits(gpu):
+    shapes = {p[3:5] for p in PLANS}
+    assert shapes == {(mt, nt) for mt in range(1, 6) for nt in (1, 2)}
+    gy = [_plan(gpu, d, True, N, True, 1, 2 * n * n if d == 2 else 6 * n ** 3)[3] for d, N, n, *_ in PLANS]
+    assert min(gy) == 1 and sum(g > 1 for g in gy) >= 5
+
+
+# p.Ap with several m-tiles, two n-tiles and a row split: history against the oracle's
+@pytest.mark.parametrize("dim,N,n", [(2, 3, 90), (2, 10, 22), (3, 4, 14), (3, 8, 7)])
+def test_simplex_plans_inside_cg(gpu, dim, N, n):
+    gm = _simplex_mesh(gpu, dim, N, n)
+    S = gpu.BP(gm, precon="JACOBI")
+    b, dinv = S.rhs("RANDOM", 0).download(), 1.0 / S.diagonal().download()
+    x = gpu.DeviceBuffer.from_host(np.zeros(gm.Ngather))
+    st, hr, _ = S.solve(x, gpu.DeviceBuffer.from_host(b), tol=0.0, maxit=6)
+    rows, cols = gm.array("rowStarts"), gm.array("colIds")
+    r, p, ho = b.copy(), None, []
+    for k in range(6):
+        z = dinv * r
+        rz = r @ z
+        p = z if p is None else z + rz / rz0 * p
+        Ap = np.add.reduceat(_simplex_reference(gm, p).reshape(-1)[cols], rows[:-1])
+        r, rz0 = r - rz / (p @ Ap) * Ap, rz
+        ho.append(np.linalg.norm(r))
+    assert st.iterations == 6 and np.max(np.abs(hr - ho) / ho) < 1e-10
