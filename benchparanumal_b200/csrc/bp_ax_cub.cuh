@@ -87,34 +87,47 @@ static_assert(kCubTable * sizeof(double) <= 64 * 1024, "constant table exceeds t
 static __constant__ CubReal c_cub[kCubTable];
 
 // Slots per block, registers a thread may take and unrolling, by the points G
-// per direction (sweeps over all degrees, 10^3..60^3 boxes, both precisions;
-// GB/s of the byte model).  Several slots only where one leaves the block
-// small (a mass element of 9 threads: 28 slots 2940 GB/s, 7 slots 1950; the
-// counts divide by three there, so that the fields of an element share a
-// block's L1) or a
-// warp half empty (G = 6: 36 threads).  Registers: the least that does not
-// spill, for more resident blocks (FP64 stiffness G = 9: 96 registers 4002,
-// 80 3726 GB/s; G = 10: 96 3855, 128 3620).  Outputs of a line are unrolled but
-// for FP64 G = 13 and 17 and FP32 G = 12..14 (spills: FP32 G = 13 1979 against
-// 2024 GB/s rolled by three); the flux loop runs three points at a time, the
-// mass columns as a whole (FP64 G = 11: 3083 against 2946 GB/s by three),
-// except where that spills (G = 16: 350 against 62 us).
+// per direction (sweeps over 8,000 to 2.5 million nodes, one and three fields,
+// with and without q.Aq; times below are the geometric mean over these).
+// Several slots only where one leaves the block small (a mass element of 9
+// threads: 28 slots 2940 GB/s, 7 slots 1950; curved, 14 slots take 0.97 of 21's
+// time, affine 1.19; FP64 stiffness 0.92 with 48 registers) or a warp half empty
+// (G = 6: 36 threads).  Registers: few, for more resident blocks, where a few
+// spilled values cost less than these give (FP64 stiffness G = 9: 96 registers
+// 4002, 80 3726 GB/s; G = 10: 96 3855, 128 3620).  Outputs of a line are unrolled
+// but for FP64 G = 13 and 17 and the curved FP32 G = 13 (spills).  The flux loop runs three points at a time in FP64 and, in
+// FP32, as a whole up to G = 7 (0.87-0.95 of the time of three at a time, or of
+// one at a time at G = 6).  FP32 G = 12: unrolled outputs 0.82 (curved) and 0.70
+// (affine) of rolled ones; G = 13 and 14, with 80 and 128 registers, 0.85-0.95
+// and 0.83-0.89.  The mass columns run as a whole (FP64 G = 11: 3083 against
+// 2946 GB/s by three), except where that spills (G = 16: 350 against 62 us).
 template <int NQ, int FORM>
 struct CubRule {
   static constexpr bool CURVED = (FORM == CUB_MASS || FORM == CUB_STIFF);
   static constexpr bool STIFF = (FORM == CUB_STIFF_AFFINE || FORM == CUB_STIFF);
   static constexpr bool D = sizeof(CubReal) == 8;
   static constexpr int G = CURVED ? NQ + 1 : NQ;
-  static constexpr int EPB = STIFF ? (G == 2 ? 24 : G == 3 ? 21 : G == 4 ? 6 : G <= 6 ? 5 : G == 8 && D ? 2 : 1)
-                                   : (G == 2 ? 24 : G == 3 ? 21 : G == 4 ? 12 : G <= 6 ? 5 : G == 7 ? 3 : G == 8 ? 2 : 1);
+  static constexpr int EPB =
+      G == 2   ? 24
+      : G == 3 ? (STIFF || CURVED ? 14 : 21)
+      : STIFF  ? (G == 4 ? (D ? 6 : 8) : G == 5 ? 5 : G == 6 ? (D ? 5 : 3) : G == 8 && D ? 2 : 1)
+               : (G == 4 ? (CURVED ? 8 : 12) : G <= 6 ? 5 : G == 7 ? 3 : G == 8 ? 2 : 1);
   static constexpr int WARPS = (G * G * EPB + 31) / 32;
-  static constexpr int REGS = !D ? (G <= 7 ? 48 : 3 * G + 26) : !STIFF ? 4 * G + 24 : G <= 6 ? 64 : G == 7 ? 80 : G <= 13 ? 100 : G <= 16 ? 128 : 170;
+  static constexpr int REGS = !D       ? (G <= 7 ? 48 : G == 13 && STIFF ? 80 : G == 14 && STIFF ? 128 : 3 * G + 26)
+                              : !STIFF ? 4 * G + 24
+                              : G == 3 ? 48
+                              : G <= 6 ? 64
+                              : G == 7 ? 80
+                              : G <= 13 ? 100
+                              : G <= 16 ? 128 : 170;
   static constexpr int minb(bool dot) {   // resident blocks to allow for (the q.Aq form takes 8 registers more)
     const int n = 65536 / (WARPS * 32 * (REGS + (dot ? 8 : 0)));
     return n < 1 ? 1 : n * WARPS > 64 ? 64 / WARPS : n > 32 ? 32 : n;
   }
-  static constexpr int UN = STIFF && (D ? G == 13 || G == 17 : G >= 12 && G <= 14) ? 3 : G;
-  static constexpr int UK = STIFF ? (G == 6 ? 1 : 3) : G == 16 ? 3 : G;
+  static constexpr int UN = !STIFF ? G : D ? (G == 13 || G == 17 ? 3 : G) : (G == 13 && CURVED ? 4 : G);
+  static constexpr int UK = !STIFF ? (G == 16 ? 3 : G)
+                            : D    ? (G == 6 ? 1 : 3)
+                                   : (G <= 7 ? G : G == 13 || G == 14 ? 4 : 3);
 };
 
 // One element (of one field) per slot of G x G threads, EPB slots per block.

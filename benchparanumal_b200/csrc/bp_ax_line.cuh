@@ -253,16 +253,27 @@ struct LinesShape {
   static constexpr int RS = (NQ % 2 || NQ == 6 || NQ == 10 || NQ == 14) ? NQ : NQ + 1;
   static constexpr int PL = NQ * RS + (NQ == 6 ? 1 : NQ == 7 ? 5 : NQ == 10 ? 5 : NQ == 14 ? 9 : NQ == 16 ? 15 : 0);
   static constexpr int FIELD = NQ * PL;
-  static constexpr int EPB = NQ == 2 ? 24 : NQ == 3 ? 21 : NQ == 4 ? 6 : NQ <= 6 ? 5 : NQ == 8 && D ? 2 : 1;
+  // slots, registers and unrolling from sweeps over 8,000 to 2.5 million nodes,
+  // both factor storages, one and three fields, with and without p.Ap (times are
+  // the geometric mean over these): FP64 Nq = 5 three slots and the flux loop as
+  // a whole 0.93 of five slots by three points; Nq = 2 with p.Ap 40 registers 0.83
+  // of 64; FP32 the flux loop as a whole at Nq = 4, 11, 13 0.92-0.96; Nq = 12
+  // outputs unrolled 0.89
+  static constexpr int EPB = NQ == 2 ? 24 : NQ == 3 ? 21 : NQ == 4 ? 6 : NQ == 5 ? (D ? 3 : 5) : NQ == 6 ? 5 : NQ == 8 && D ? 2 : 1;
   static constexpr int WARPS = (G2 * EPB + 31) / 32;
   static constexpr int THREADS = WARPS * 32;   // whole warps; the last threads own no line
-  // registers a thread may take: the least that does not spill, for more resident blocks
-  static constexpr int REGS = !D ? (NQ <= 7 ? 48 : 3 * NQ + 26) : NQ <= 6 ? 64 : NQ == 7 ? 80 : NQ <= 13 ? 100 : 128;
-  static constexpr int minb(bool dot) {   // resident blocks to allow for (the p.Ap form takes 8 registers more)
-    const int n = 65536 / (THREADS * (REGS + (dot ? 8 : 0)));
+  // registers a thread may take: few, for more resident blocks, where spills cost less than these give
+  static constexpr int regs(bool dot) {   // (the p.Ap form takes 8 more)
+    if (D && NQ == 2) return dot ? 48 : 64;
+    if (!D && NQ == 12) return dot ? 70 : 96;
+    return (!D ? (NQ <= 7 ? 48 : 3 * NQ + 26) : NQ <= 6 ? 64 : NQ == 7 ? 80 : NQ <= 13 ? 100 : 128) + (dot ? 8 : 0);
+  }
+  static constexpr int minb(bool dot) {   // resident blocks to allow for
+    const int n = 65536 / (THREADS * regs(dot));
     return n < 1 ? 1 : n * WARPS > 64 ? 64 / WARPS : n > 32 ? 32 : n;
   }
-  static constexpr int UN = D ? (NQ == 13 ? 3 : NQ) : (NQ >= 12 && NQ <= 14 ? 3 : NQ);
+  static constexpr int UN = D ? (NQ == 13 ? 3 : NQ) : (NQ == 13 ? 4 : NQ == 14 ? 3 : NQ);
+  static constexpr int UK = D ? (NQ == 5 ? NQ : 3) : (NQ == 4 || NQ == 11 || NQ == 13 ? NQ : 3);   // flux loop
   static constexpr int SLOT = line_slot(NQ);
   static constexpr size_t SMEM0 = sizeof(LineReal) * (size_t)3 * FIELD * EPB;
   static constexpr size_t SMEM = SMEM0 < sizeof(double) * THREADS ? sizeof(double) * THREADS : SMEM0;
@@ -296,7 +307,7 @@ ax_lines_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementL
   using F = LineReal;
   using Sh = LinesShape<NQ>;
   using V2 = typename std::conditional<sizeof(F) == 8, double2, float2>::type;
-  constexpr int G2 = Sh::G2, NP = Sh::NP, RS = Sh::RS, PL = Sh::PL, EPB = Sh::EPB, UN = Sh::UN;
+  constexpr int G2 = Sh::G2, NP = Sh::NP, RS = Sh::RS, PL = Sh::PL, EPB = Sh::EPB, UN = Sh::UN, UK = Sh::UK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int slot = EPB == 1 || threadIdx.x >= G2 * EPB ? 0 : threadIdx.x / G2;
   const int t = threadIdx.x - slot * G2;      // >= G2: no line
@@ -348,7 +359,7 @@ ax_lines_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementL
       u[n] = U[tcol + n * PL];
       acc[n] = 0;
     }
-#pragma unroll 3
+#pragma unroll UK
     for (int k = 0; k < NQ; ++k) {
       F g[6], w;
       if (AFFINE) {
