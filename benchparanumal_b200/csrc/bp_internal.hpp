@@ -5,7 +5,6 @@
 
 #include <atomic>
 #include <cstdint>
-#include <cstdlib>
 #include <functional>
 #include <mutex>
 #include <string>

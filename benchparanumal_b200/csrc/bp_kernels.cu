@@ -177,10 +177,9 @@ ax_pencil_kernel(int Nelements, const int32_t* __restrict__ elementList, const i
   if (DOT) fuse_pap(pdot, fuse, s_red);
 }
 
-// Kernel variant of the element operator: stored factors use the TMA-staged
-// kernel where it applies and the line-per-thread kernel (bp_ax_line.cuh)
-// elsewhere; affine factors the tensor-core kernel at Nq = 16 (bp_ax_mma.cu),
-// else the line kernel in FP32 and the register-pencil kernel in FP64.
+// Kernel variant of the element operator, chosen by the autotuner among the
+// TMA-staged, line-per-thread (bp_ax_line.cuh), register-pencil and, for affine
+// factors at Nq = 16, tensor-core (bp_ax_mma.cu) kernels: see ax_forms.
 // BP_AX_VARIANT=pencil, =line, =tma or =mma in the environment selects that
 // kernel wherever it applies (for comparisons).
 int ax_variant() {   // read at every launch, so a process (a test) can switch forms
@@ -191,7 +190,7 @@ int ax_variant() {   // read at every launch, so a process (a test) can switch f
          s == "rb" ? AX_RB : AX_AUTO;
 }
 
-// The register-pencil form (FP64 affine default; any configuration)
+// The register-pencil form (any configuration and factor alignment)
 template <int NQ, class F>
 static int launch_pencil(const bp_ax_desc_t& d, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                          const F* wJ, const F* ggeo, const F* gllw, const F* D, F lambda, const F* q, F* Aq,
@@ -246,13 +245,17 @@ static int launch_ax_form(int form, const bp_ax_desc_t& d, int32_t Nelements, co
   }
 }
 
-// The forms that may serve d, the measured static choice first (40^3 or 24^3
-// boxes): stored factors the TMA kernel where it applies (even Nq), else the
-// line kernel (FP32 mixed BP5 p=10: 0.61 vs 1.15 s pencil; FP64 BK5 p=6 0.6
-// vs 0.7 ms); affine factors the tensor-core kernel at Nq = 16 (BK6 p=15 FP64
-// 2.3 vs 7.5 ms, FP32 1.4 vs 4.0 ms), else the line kernel in FP32 and the
-// pencil kernel in FP64 (BK5 p=7 0.6 vs 0.8 ms).  The autotuner measures them
-// all on first use and keeps the fastest.
+// The forms that may serve d, the static choice first: what an untuned
+// configuration gets under a stream capture or with BP_AUTOTUNE=0 (stored factors
+// the TMA kernel where it applies, else the line kernel; affine factors the
+// tensor-core kernel at Nq = 16, else the line kernel in FP32 and the pencil
+// kernel, which reads D and gllw from the arguments, in FP64).  The autotuner
+// measures them all on first use outside a capture and keeps the fastest.  The
+// static order predates the present line form, which the tuner prefers on large
+// meshes (2.5 million nodes, us): stored FP64 p=7 63 (TMA) against 60, p=15 95
+// against 72, three fields p=7 175 against 126; affine FP64 p=7 62 (pencil)
+// against 39, p=14 248 against 53; on small ones (60,000 nodes, launch and
+// constant copy included) the pencil form below p=6 (p=3 12.9 TMA, 9.9 line, 6.9).
 template <int NQ, class F>
 static std::vector<int> ax_forms(const bp_ax_desc_t& d) {
   std::vector<int> f;

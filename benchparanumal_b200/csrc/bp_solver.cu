@@ -3,7 +3,7 @@
 // libs/core/linearSolverCG.cpp:62-156).
 //
 // CG runs with every scalar on the device.  One iteration is four kernels
-// (three on small meshes, where the gather forms alpha itself: kFoldParts):
+// (three where the operator leaves few partials and the gather forms alpha: kFoldParts):
 //   cg_direction_kernel     x += alpha_{k-1} p_{k-1} (deferred),  p = z + beta p
 //   element operator        AqL = A_e p, and block partials of p.Ap = sum_e p_e.(A_e p_e)
 //   cg_alpha_kernel         p.Ap from the partials, alpha = rho / p.Ap
@@ -241,16 +241,22 @@ cg_alpha_kernel(int nparts, const double* __restrict__ parts, CgScalars* sc, dou
 // programmatic launch): an SM keeps its split between L1 and shared memory
 // while blocks follow one another, and a gather that slips in behind an
 // operator with 224 KB of shared memory per SM is left without the L1 that
-// its indices and shared lines need (packed p=7 22x24x23 to 1e-8: 254 ms
-// against 218; a gather denied its L1 outright 253, denied shared memory 374).
+// its indices and shared lines need (packed p=7 22x24x23 to 1e-8: behind the line
+// form 260 ms against 220, behind the TMA form 230 either way).  One right-hand
+// side: the same within 3%, but FP64 p=1 at 3 million elements 586 us an
+// iteration against 557.
 //
-// Up to this many block partials every block of the gather-update
-// adds them for itself (the same order in each, so the same alpha) and the
-// alpha kernel is left out: a read of at most 8 KB from L2 against a launch
-// with its own grid reduction (FP64, 100 iterations: p=4 16^3 2.75 -> 2.64 ms,
-// p=10 5^3 2.51 -> 1.83 ms; four packed lanes, four sums in each block, lose:
-// p=4 10^3 to 1e-8 6.43 -> 6.69 ms, and keep the kernel).  Beyond, the
-// reads by a thousand blocks cost more than the kernel they save.
+// Up to this many block partials every block of the gather-update adds them
+// for itself (the same order in each, so the same alpha) and the alpha kernel is
+// left out: a read of at most 8 KB from L2 against a launch with its own grid
+// reduction.  The rule counts blocks of the operator, not rows.  Measured in one
+// process, p = 1..15, 1e4 to 3e6 rows, time per iteration of three kernels by
+// four: FP64 0.69-0.98; FP32 0.63-1.00 up to a million rows, 1.04 at 1000
+// elements of p=15 (3.3 million rows).  Above 1024 partials: FP64 0.92-0.98 up to
+// 1e5-3e5 rows, then even (p=1 1.18); FP32 loses 2-10% from 1e6 rows on.
+// Launched programmatically the folded gather gains up to a third of the
+// iteration up to 1e5 rows and changes nothing beyond.  Four packed lanes, four
+// sums in each block, lose (p=4 10^3 to 1e-8 6.43 -> 6.69 ms) and keep the kernel.
 constexpr int kFoldParts = 1024;
 
 // p.Ap from the operator's block partials, the same bits in every thread of

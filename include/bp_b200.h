@@ -97,7 +97,11 @@ typedef struct bp_ax_desc {
    ggeo: non-affine [E*Np*6] node-major G00,G01,G02,G11,G12,G22 with the GLL
    weights folded in, wJ [E*Np]; affine ggeo [E*6], wJ [E] (weights applied in
    the kernel from gllw).  D: [Nq*Nq] row-major, D[i*Nq+m] = l_m'(r_i).
-   q: gathered vector; Aq: E-vector [E*Np*Nfields], layout e*Np*Nf + f*Np + n. */
+   q: gathered vector; Aq: E-vector [E*Np*Nfields], layout e*Np*Nf + f*Np + n.
+   D and gllw may pass through a constant table with one slot per degree and
+   precision, filled in stream order: Hex3D calls of one degree that can overlap
+   on different streams must pass the same D and gllw (a degree has one such pair
+   on GLL nodes), and so must the over-integrated calls their matrices. */
 int bp_ax_hex3d(const bp_ax_desc_t* desc, int32_t Nelements, const int32_t* elementList,
                 const int32_t* GlobalToLocal, const double* wJ, const double* ggeo,
                 const double* gllw, const double* D, double lambda, const double* q,
@@ -503,7 +507,7 @@ int bp_driver_main(const char* name, int argc, char** argv);
  * untimed and three timed launches each) and keeps the fastest for that
  * configuration and element-count class (floor(log2(Nelements))) on the
  * device.  Solvers launch their operator once before capturing their graphs.
- * While a stream captures, an untuned configuration takes the measured static
+ * While a stream captures, an untuned configuration takes the static
  * choice.  BP_AUTOTUNE=0 in the environment keeps the static choice.
  * ------------------------------------------------------------------------- */
 #define BP_FORM_MMA 0     /* tensor-core MMA (affine Nq = 16; packed Nq = 8) */
