@@ -255,11 +255,12 @@ struct LinesShape {
   static constexpr int FIELD = NQ * PL;
   // slots, registers and unrolling from sweeps over 8,000 to 2.5 million nodes,
   // both factor storages, one and three fields, with and without p.Ap (times are
-  // the geometric mean over these): FP64 Nq = 5 three slots and the flux loop as
-  // a whole 0.93 of five slots by three points; Nq = 2 with p.Ap 40 registers 0.83
-  // of 64; FP32 the flux loop as a whole at Nq = 4, 11, 13 0.92-0.96; Nq = 12
-  // outputs unrolled 0.89
-  static constexpr int EPB = NQ == 2 ? 24 : NQ == 3 ? 21 : NQ == 4 ? 6 : NQ == 5 ? (D ? 3 : 5) : NQ == 6 ? 5 : NQ == 8 && D ? 2 : 1;
+  // the geometric mean over these): FP64 Nq = 5 the flux loop as a whole 0.96 of
+  // three points at a time (with three slots 0.93, but then more partials: 16^3
+  // elements at p=4 would keep the alpha kernel, 100 CG iterations 2.86 against
+  // 2.66 ms); Nq = 2 with p.Ap 40 registers 0.83 of 64; FP32 the flux loop as a
+  // whole at Nq = 4, 11, 13 0.92-0.96; Nq = 12 outputs unrolled 0.89
+  static constexpr int EPB = NQ == 2 ? 24 : NQ == 3 ? 21 : NQ == 4 ? 6 : NQ <= 6 ? 5 : NQ == 8 && D ? 2 : 1;
   static constexpr int WARPS = (G2 * EPB + 31) / 32;
   static constexpr int THREADS = WARPS * 32;   // whole warps; the last threads own no line
   // registers a thread may take: few, for more resident blocks, where spills cost less than these give
