@@ -61,13 +61,14 @@ CONFIG = {"workload": WORKLOAD, "nx": NX, "ny": NX, "nz": NX, "p": P, "Ndofs": (
           "tolerance": TOL, "perturbation": PERT, "perturbation_seed": PERT_SEED, "forcing_seeds": list(range(NRHS)),
           "l2": "inputs larger than L2 (FP32 factors 0.92 GB read per packed operator apply)"}
 B200_SMS = 148
-# One launch of the packed FP32 element operator (4 rhs) on this workload,
-# captured by ncu at full size (BK5 -nx 40 -ny 40 -nz 40 -p 7 -pt 0.1 -f RANDOM
-# -fp MIXED -nr 4, one kernel, one launch): DRAM bytes read + written, and
-# shared-memory wavefronts (loads + stores).  The kernel is bound by that
-# pipe: one wavefront per SM and clock.
-AX_DRAM_BYTES = 1396588800 + 498959616
-AX_SMEM_WAVEFRONTS = 141570589
+# One launch of the packed FP32 element operator (4 rhs) on this workload, by
+# autotuner form, captured by ncu at full size (BK5 -nx 40 -ny 40 -nz 40 -p 7
+# -pt 0.1 -f RANDOM -fp MIXED -nr 4, one kernel, one launch): DRAM bytes read +
+# written (the line form's as ncu prints them, three digits), and shared-memory
+# wavefronts (loads + stores).  The TMA form is bound by that pipe: one wavefront
+# per SM and clock.
+AX_DRAM_BYTES = {"tma": 1396588800 + 498959616, "line": 1400000000 + 501090000}
+AX_SMEM_WAVEFRONTS = {"tma": 141570589, "line": 75085313}
 # kernel instantiations of the packed four-system FP32 operator, by autotuner form
 AX_KERNELS = {"tma": "ax_tma_kernel<NQ=8,NF=1,DOT=0,R=4,float,Pack<float,4>>",
               "rb": "ax_rb_kernel<NQ=8,L=4,DOT=0>",
@@ -479,7 +480,8 @@ def main():
     peak, peak_kind = read_peaks()
     achieved = ax_bytes / ax_s / 1e9
     smem_mhz = (clk or {}).get("sm_mhz") or (clk or {}).get("sm_max_mhz") or 1965.0
-    smem_bound_ms = AX_SMEM_WAVEFRONTS / (B200_SMS * smem_mhz * 1e6) * 1e3
+    smem_wf = AX_SMEM_WAVEFRONTS.get(ax_form)
+    smem_bound_ms = smem_wf / (B200_SMS * smem_mhz * 1e6) * 1e3 if smem_wf else None
     del AqL, ops, vec, invD32, own, parts, b32
 
     # free the headline's buffers before the other configurations
@@ -515,17 +517,16 @@ def main():
                          "kernel": AX_KERNELS.get(ax_form, str(ax_form)) + " (bp_ax_hex3d_f32_multi, 4 rhs)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak, "algorithmic_bytes": ax_bytes,
-                         # DRAM bytes and wavefronts were captured with ncu on the TMA form
-                         "traffic": AX_DRAM_BYTES if ax_form == "tma" else None,
+                         # captured with ncu on the forms listed
+                         "traffic": AX_DRAM_BYTES.get(ax_form),
                          "launch_ms": ax_s * 1e3,
                          "fused_direction_step": {"kernel": "bp_cg_direction_ax_f32_multi (4 rhs)",
                                                   "launch_ms": fused_s * 1e3, "algorithmic_bytes": fused_bytes,
                                                   "achieved": fused_bytes / fused_s / 1e9},
-                         # the roof that binds this kernel: shared-memory wavefronts at one per SM and clock
-                         # (clock: the median SM clock sampled during the timed step, else the maximum)
-                         "smem": {"wavefronts": AX_SMEM_WAVEFRONTS, "sm_mhz": smem_mhz,
-                                  "bound_ms": smem_bound_ms, "frac": smem_bound_ms / (ax_s * 1e3)}
-                         if ax_form == "tma" else None},
+                         # the shared-memory pipe's time: wavefronts at one per SM and clock (clock: the
+                         # median SM clock sampled during the timed step, else the maximum)
+                         "smem": {"wavefronts": smem_wf, "sm_mhz": smem_mhz, "bound_ms": smem_bound_ms,
+                                  "frac": smem_bound_ms / (ax_s * 1e3)} if smem_wf else None},
             "cpu_baseline": cpu,
             "cpu": cpu_info(),
             "configs": extras,
