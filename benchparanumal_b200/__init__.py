@@ -177,7 +177,7 @@ def lib():
             "bp_box_vertices": [ctypes.POINTER(BoxDesc), vp, vp, vp],
             "bp_ogs_check": [ctypes.c_int64, vp, i32, vp, vp],
             "bp_test_wait_timeout": [ctypes.c_int],
-            "bp_test_operator_plan": [ctypes.c_int] * 5 + [i32, vp],
+            "bp_test_operator_plan": [ctypes.c_int] * 6 + [i32, vp],
             "bp_tune_report": [i32] * 8 + [ctypes.POINTER(i32), ctypes.POINTER(i32), vp, vp, i32],
             "bp_tune_reset": [],
             "bp_operator_hex3d_noalloc": [ctypes.POINTER(AxDesc), i32, vp, vp, vp, vp, vp, vp, dbl, i32, i32, vp,

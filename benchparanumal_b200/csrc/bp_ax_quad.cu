@@ -16,16 +16,21 @@
 
 namespace bp {
 
-// The line form from the warps per SM on at which it overtakes the node form,
-// measured at 1 to 40 warps per SM, all degrees, both precisions and field
-// counts: with stored factors between 4 (p=12) and 11 (FP32 p=2), at most
-// degrees near 8 (node/line time at p=5 FP64 0.88 at 6 warps, 1.02 at 8, 1.13
-// at 16; p=8 FP32 0.83, 0.97, 1.39); affine, where the line form's loads are
-// fewer, between 2 and 5 (p=5 FP64 0.78 at 2, 0.93 at 3, 1.03 at 6).  Two
-// fields, whose factors the node form reads once, somewhat later.
-bool quad_line_form(int N, int affine, int Nfields, int32_t Nelements) {
-  const int warps = affine ? 2 + Nfields : 6 + 2 * Nfields;
-  return (int64_t)Nelements * Nfields >= (int64_t)warps * sm_count() * (32 / (N + 1));
+// The line form from the warps per SM on at which it overtakes the node form:
+// tenths of a warp by degree, measured at 1 to 40 warps per SM over all degrees,
+// precisions, factor storages and field counts (1200 meshes; the form chosen
+// takes 1.003 of the better one's time on average, 1.16 at the most, where one
+// figure for all degrees, 8 warps stored and 3 affine, took 1.02 and 3.4).  The
+// line form comes late at low degrees in FP32 (stored p=2 at 8 warps 3.3 us against
+// 2.9) and early at high ones, where the node form's block holds one element
+// (FP64 p=14 at 8 warps 10 us against 35).  Affine, its loads are fewer and it
+// comes sooner; with two fields, whose factors the node form reads once, later.
+bool quad_line_form(int N, int affine, int Nfields, int bytes, int32_t Nelements) {
+  static const short stored64[15] = {80, 100, 80, 80, 80, 40, 60, 50, 60, 50, 60, 35, 40, 15, 35};
+  static const short stored32[15] = {80, 140, 100, 100, 90, 70, 70, 80, 60, 80, 70, 60, 50, 40, 40};
+  static const short aff[15] = {40, 60, 40, 30, 40, 20, 30, 30, 30, 30, 35, 30, 25, 15, 25};
+  const int hundredths = (affine ? aff : bytes == 8 ? stored64 : stored32)[N - 1] * (Nfields == 1 ? 10 : affine ? 12 : 13);
+  return (int64_t)100 * Nelements * Nfields >= (int64_t)hundredths * sm_count() * (32 / (N + 1));
 }
 
 namespace {
@@ -274,7 +279,7 @@ static int launch_quad_nq(const bp_ax_desc_t& d, int32_t Nelements, const int32_
                           const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks) {
   using Sh = QuadShape<NQ>;
   const CgFuse Fz = fuse ? *fuse : CgFuse{};
-  if (!quad_line_form(d.N, d.affine, d.Nfields, Nelements)) {
+  if (!quad_line_form(d.N, d.affine, d.Nfields, (int)sizeof(F), Nelements)) {
     using Nd = QuadNodeShape<NQ>;
     const dim3 grid((Nelements + Nd::EPB - 1) / Nd::EPB), block(NQ, NQ, Nd::EPB);
     if (nblocks) *nblocks = (int)grid.x;

@@ -380,15 +380,16 @@ struct SimplexMmaPlan {
 //
 // A block alone on its SM takes the k steps of its rounds, each with its tile
 // products, fragment loads and a latency, after the gather of its q tile in
-// batches of dependent loads.  The n blocks of the busiest SM follow one
-// another at the pace of the more limiting of their residency (registers or
-// shared memory) and of the SM's DMMA and load pipes.  The weights (in DMMA
-// issue slots) are fitted to 6,500 timings: every plan at 199 problems, triangles
-// p = 3..15 and tetrahedra p = 2..12, 6 to 400,000 elements.  Over these the
-// chosen plan takes 1.024 of the best plan's time on average.  The rule before
-// (rounds times the step, times the waves beyond three blocks per SM) took 1.07
-// and lost to one thread per node at 700-2,100 elements: tetrahedra p=8, 750:
-// 49 us against 44 there and 30 now; p=5, 2,058: 22, 20, 14.
+// batches of dependent loads.  The n blocks of an SM (halfway between the busiest
+// and the average one) follow one another at the pace of the more limiting of
+// their residency (registers or shared memory) and of the SM's DMMA and load
+// pipes.  The weights (in DMMA issue slots) are fitted to the timings of every
+// plan at 592 problems, triangles p = 3..15 and tetrahedra p = 2..12, 6 to 400,000
+// elements.  Over these the chosen plan takes 1.028 of the best plan's time on
+// average, a tenth of them more than 1.10.  The rule before (rounds times the
+// step, times the waves beyond three blocks per SM) took 1.11 and lost to one
+// thread per node at 700-2,100 elements: tetrahedra p=8, 750: 49 us against 44
+// there and 30 now; p=5, 2,058: 22, 20, 14.
 static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms) {
   constexpr int regs[5] = {72, 96, 128, 128, 168};   // registers a thread of the kernel takes, by mt
   const int tiles = (Np + 7) / 8;
@@ -403,13 +404,14 @@ static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms) {
         const int bx = (E + p.eb() - 1) / p.eb();
         p.gy = std::max(1, std::min(sets, 2 * sms / bx));
         const int rounds = (sets + p.gy - 1) / p.gy;
-        const double n = (bx * (int64_t)p.gy + sms - 1) / sms;
+        const int64_t blocks = bx * (int64_t)p.gy;
+        const double n = 0.5 * ((blocks + sms - 1) / sms) + 0.5 * std::max((double)blocks / sms, 1.0);
         const double steps = (double)rounds * C * ((Np + 3) / 4);
         const double gathers = p.eb() * ((Np + 3) / 4 * 4) / (6.0 * 32 * kMmaWarps);
         const int resident = (int)std::min<size_t>(65536 / (regs[mt - 1] * 32 * kMmaWarps),
                                                    227 * 1024 / (p.smem(Np) + 1024));
-        const double alone = steps * (mt * nt + 0.7 * mt + 3.4 * nt + 7) + 60 * std::ceil(gathers);
-        const double pipes = steps * (0.8 * mt * nt + 0.4 * mt) + 11 * gathers;
+        const double alone = steps * (mt * nt + 0.9 * mt + 3.6 * nt + 8) + 40 * std::ceil(gathers);
+        const double pipes = steps * (mt * nt + 0.2 * mt + 0.05) + 4 * gathers;
         const double c = alone + (n - 1) * std::max(alone / resident, pipes);
         if (c < cost) {
           cost = c;

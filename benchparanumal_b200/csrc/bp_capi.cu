@@ -126,13 +126,15 @@ const char* bp_version(void) { return "benchparanumal_b200 0.1 (sm_100a)"; }
 
 int bp_test_wait_timeout(int withhold_slice) { return tma_wait_test(withhold_slice); }
 
-int bp_test_operator_plan(int dim, int simplex, int N, int affine, int Nfields, int32_t Nelements, int32_t* plan) {
-  if (!plan || Nelements < 1 || N < 1 || N > 15 || Nfields < 1 || (dim != 2 && dim != 3) || (dim == 3 && !simplex))
+int bp_test_operator_plan(int dim, int simplex, int N, int affine, int Nfields, int bytes, int32_t Nelements,
+                          int32_t* plan) {
+  if (!plan || Nelements < 1 || N < 1 || N > 15 || Nfields < 1 || (bytes != 8 && bytes != 4) ||
+      (dim != 2 && dim != 3) || (dim == 3 && !simplex))
     return fail(BP_ERROR_ARG, "bp_test_operator_plan: no such operator");
   if (simplex) {
     simplex_plan(dim, N, Nelements, plan);
   } else {
-    plan[0] = quad_line_form(N, affine, Nfields, Nelements) ? 1 : 0;
+    plan[0] = quad_line_form(N, affine, Nfields, bytes, Nelements) ? 1 : 0;
     plan[1] = plan[2] = plan[3] = 0;
   }
   return BP_SUCCESS;

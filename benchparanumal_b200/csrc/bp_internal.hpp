@@ -450,7 +450,7 @@ int launch_ax_mma_packed(int pk, const bp_ax_desc_t& d, int32_t Nelements, const
 // Quad2D forms (bp_ax_quad.cu): the BP5/BP6 element operator (FP64 and FP32;
 // 1 with a fused direction update, which it does not take), the forcing, the
 // lumped mass and the element diagonal
-bool quad_line_form(int N, int affine, int Nfields, int32_t Nelements);   // rather than the node form
+bool quad_line_form(int N, int affine, int Nfields, int bytes, int32_t Nelements);   // rather than the node form
 int launch_ax_quad(const bp_ax_desc_t& d, int32_t Nelements, const int32_t* elementList, const int32_t* G2L,
                    const double* wJ, const double* ggeo, const double* gllw, const double* D, double lambda,
                    const double* q, double* Aq, const int* skip, const CgFuse* fuse, cudaStream_t s, int* nblocks);

@@ -555,7 +555,8 @@ int bp_test_wait_timeout(int withhold_slice);
    for the line form, 0 for the node form.  Simplex: 8-node tiles and 8-element
    tiles per warp, warps along the nodes, blocks along the nodes (all 0 below 8
    nodes per element, where a thread serves a node). */
-int bp_test_operator_plan(int dim, int simplex, int N, int affine, int Nfields, int32_t Nelements, int32_t* plan);
+int bp_test_operator_plan(int dim, int simplex, int N, int affine, int Nfields, int precision_bytes,
+                          int32_t Nelements, int32_t* plan);
 
 #ifdef __cplusplus
 }

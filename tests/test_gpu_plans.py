@@ -16,9 +16,9 @@ def _rel(a, b):
     return float(np.max(np.abs(a - b)) / max(np.max(np.abs(b)), 1e-300))
 
 
-def _plan(gpu, dim, simplex, N, affine, nf, n):
+def _plan(gpu, dim, simplex, N, affine, nf, n, precision_bytes=8):
     p = np.zeros(4, np.int32)
-    gpu._check(gpu.lib().bp_test_operator_plan(dim, int(simplex), N, int(affine), nf, n, p.ctypes.data))
+    gpu._check(gpu.lib().bp_test_operator_plan(dim, int(simplex), N, int(affine), nf, precision_bytes, n, p.ctypes.data))
     return tuple(int(v) for v in p)
 
 
@@ -42,14 +42,14 @@ def _quad_reference(gm, q):
 
 
 def _quad_mesh(gpu, N, affine, nf, line):
-    """The smallest box of nx x (nx + 1) elements that takes the line form, or 3 x 2."""
+    """The smallest box of nx x (nx + 1) elements that takes the line form in both precisions, or 3 x 2."""
     nx, ny = 3, 2
     if line:
-        while not _plan(gpu, 2, False, N, affine, nf, nx * ny)[0]:
+        while not all(_plan(gpu, 2, False, N, affine, nf, nx * ny, b)[0] for b in (8, 4)):
             nx += 1
             ny = nx + 1
     gm = gpu.Mesh(nx, ny, 1, N=N, affine=affine, Nfields=nf, pert=0.0 if affine else 0.1, dim=2)
-    assert _plan(gpu, 2, False, N, affine, nf, gm.E)[0] == int(line)
+    assert all(_plan(gpu, 2, False, N, affine, nf, gm.E, b)[0] == int(line) for b in (8, 4))
     return gm
 
 
@@ -117,12 +117,12 @@ def _simplex_reference(gm, q):
 # (dim, degree, cells per direction) and the 8-node tiles, 8-element tiles and warps
 # along the nodes of the plan on 148 SMs.  The permuted list leaves elements out,
 # and the last tile partly empty in the one list or the other.
-PLANS = [(2, 3, 1, 1, 1, 1), (2, 6, 1, 1, 1, 2), (2, 9, 1, 1, 1, 4), (2, 3, 100, 1, 2, 2), (2, 6, 90, 1, 2, 4),
-         (2, 3, 35, 2, 1, 1), (2, 7, 22, 2, 1, 2), (2, 10, 16, 2, 1, 4), (2, 3, 90, 2, 2, 1), (2, 6, 140, 2, 2, 2),
-         (2, 9, 70, 2, 2, 4), (2, 5, 40, 3, 1, 1), (2, 7, 29, 3, 1, 2), (2, 10, 22, 3, 1, 4), (2, 10, 55, 3, 2, 1),
-         (2, 15, 35, 3, 2, 2), (3, 8, 7, 3, 2, 4), (2, 15, 29, 4, 1, 1), (2, 9, 55, 4, 1, 2), (3, 15, 3, 4, 1, 4),
-         (2, 6, 180, 4, 2, 1), (3, 8, 8, 4, 2, 2), (3, 9, 7, 4, 2, 4), (3, 7, 6, 5, 1, 1), (3, 9, 5, 5, 1, 2),
-         (2, 15, 23, 5, 1, 4), (3, 4, 14, 5, 2, 1), (2, 10, 60, 5, 2, 2), (2, 15, 43, 5, 2, 4)]
+PLANS = [(2, 3, 1, 1, 1, 1), (2, 6, 1, 1, 1, 2), (2, 9, 1, 1, 1, 4), (2, 4, 110, 1, 2, 2), (2, 6, 90, 1, 2, 4),
+         (2, 3, 44, 2, 1, 1), (2, 6, 33, 2, 1, 2), (2, 13, 17, 2, 1, 4), (2, 3, 90, 2, 2, 1), (2, 6, 110, 2, 2, 2),
+         (2, 9, 70, 2, 2, 4), (2, 5, 40, 3, 1, 1), (2, 7, 31, 3, 1, 2), (2, 10, 23, 3, 1, 4), (2, 10, 49, 3, 2, 1),
+         (2, 15, 35, 3, 2, 2), (3, 8, 7, 3, 2, 4), (2, 15, 29, 4, 1, 1), (3, 5, 9, 4, 1, 2), (2, 13, 30, 4, 1, 4),
+         (3, 8, 8, 4, 2, 2), (3, 9, 7, 4, 2, 4), (2, 13, 28, 5, 1, 1), (2, 11, 34, 5, 1, 2), (2, 15, 31, 5, 1, 4),
+         (3, 4, 14, 5, 2, 1), (2, 10, 60, 5, 2, 2), (2, 15, 43, 5, 2, 4)]
 
 
 def _simplex_mesh(gpu, dim, N, n):
