@@ -93,9 +93,11 @@ ax_quad_kernel(int Nelements, int Nfields, const int32_t* __restrict__ elementLi
   const int lane = threadIdx.x & 31, sl = lane / NQ;
   const bool on = sl < SPW;                               // the last lanes own no line
   const int slot = (threadIdx.x >> 5) * SPW + (on ? sl : 0), x = on ? lane - sl * NQ : 0;
-  const int64_t v = (int64_t)blockIdx.x * Sh::EPB + slot;  // element-major (element, field); past 2^31 with two fields
-  const bool valid = on && v < (int64_t)Nelements * Nfields;
-  const int eidx = (int)(v >> (Nfields - 1)), f = (int)v & (Nfields - 1);   // one or two fields
+  // element-major (element, field): one or two fields of fewer than 2^31 elements
+  // are counted in 32 bits (in 64 the p=7 curved case took 257 us against 251)
+  const unsigned v = blockIdx.x * Sh::EPB + slot;
+  const bool valid = on && v < (unsigned)Nelements * (unsigned)Nfields;
+  const int eidx = (int)(v >> (Nfields - 1)), f = (int)(v & (Nfields - 1));
   const int e = valid ? elementList[eidx] : 0;
   const size_t lbase = ((size_t)e * Nfields + f) * NP;
   const F* const ge = ggeo + 3 * (size_t)e * (AFFINE ? 1 : NP);
