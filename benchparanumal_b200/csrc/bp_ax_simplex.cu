@@ -375,26 +375,34 @@ struct SimplexMmaPlan {
   size_t smem(int Np) const { return sizeof(double) * (size_t)eb() * simplex_kp(Np); }
 };
 
-// The plan with the least estimated time.  A batch that leaves the chip idle
-// spreads its rows over blockIdx.y, to at most about two blocks per SM.
+// A batch that leaves the chip idle spreads its rows over blockIdx.y, to at most
+// about two blocks per SM.  Two estimates of a plan's time:
 //
-// A block alone on its SM takes the k steps of its rounds, each with its tile
-// products, fragment loads and a latency, after the gather of its q tile in
-// batches of dependent loads.  The n blocks of an SM (halfway between the busiest
-// and the average one) follow one another at the pace of the more limiting of
-// their residency (registers or shared memory) and of the SM's DMMA and load
-// pipes.  The weights (in DMMA issue slots) are fitted to the timings of every
-// plan at 592 problems, triangles p = 3..15 and tetrahedra p = 2..12, 6 to 400,000
-// elements.  Over these the chosen plan takes 1.028 of the best plan's time on
-// average, a tenth of them more than 1.10.  The rule before (rounds times the
-// step, times the waves beyond three blocks per SM) took 1.11 and lost to one
-// thread per node at 700-2,100 elements: tetrahedra p=8, 750: 49 us against 44
-// there and 30 now; p=5, 2,058: 22, 20, 14.
-static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms) {
-  constexpr int regs[5] = {72, 96, 128, 128, 168};   // registers a thread of the kernel takes, by mt
+// rough: the rounds of row sets a warp runs, times the tile products, fragment
+// loads and latency of a k step, times the waves beyond three blocks per SM.
+//
+// fine: a block alone on its SM takes the k steps of its rounds, each with its
+// tile products, fragment loads and a latency, after the gather of its q tile in
+// batches of dependent loads; the n blocks of an SM (between the average one and
+// the busiest) follow one another at the pace of the more limiting of their
+// residency (registers or shared memory) and of the SM's DMMA and load pipes.
+// Weights in DMMA issue slots, fitted to the timings of every plan at 985
+// problems, triangles p = 3..15 and tetrahedra p = 2..12, 6 to 400,000 elements,
+// with and without p.Ap.
+//
+// The fine estimate decides where the roughly best plan splits the rows (it
+// ranks splits poorly); elsewhere it has to put another plan 8% below that one.
+// Over the 985 problems this takes 1.031 of the best plan's time on average, 297
+// of them over 5% faster than the rough choice alone (which takes 1.11, and at
+// 700-2,100 elements more than one thread per node: tetrahedra p=8, 750: 49 us
+// against 44 there and 30 now; an FP64 CG iteration at p=7, 2,058: 74, 56 and 51),
+// 6 over 5% slower, 1.10 at the most.  The fine estimate alone: 1.028, but 38
+// slower, up to 1.39.
+static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms, bool dot) {
   const int tiles = (Np + 7) / 8;
-  SimplexMmaPlan best{1, 1, 1, 1};
-  double cost = 1e300;
+  const double steps1 = C * ((Np + 3) / 4);
+  SimplexMmaPlan rough{1, 1, 1, 1}, fine = rough;
+  double rough_cost = 1e300, rough_fine = 1e300, fine_cost = 1e300;
   for (int nt = 2; nt >= 1; --nt)
     for (int wm = 1; wm <= kMmaWarps; wm *= 2)
       for (int mt = 1; mt <= 5; ++mt) {
@@ -405,20 +413,30 @@ static SimplexMmaPlan simplex_mma_plan(int C, int Np, int32_t E, int sms) {
         p.gy = std::max(1, std::min(sets, 2 * sms / bx));
         const int rounds = (sets + p.gy - 1) / p.gy;
         const int64_t blocks = bx * (int64_t)p.gy;
-        const double n = 0.5 * ((blocks + sms - 1) / sms) + 0.5 * std::max((double)blocks / sms, 1.0);
-        const double steps = (double)rounds * C * ((Np + 3) / 4);
+        const double per_sm = (double)blocks / sms;
+        const double r = std::max(per_sm / 3, 1.0) * rounds * (mt * nt + 0.6 * mt + 0.3 * nt + 1.5);
+
+        // registers a thread of the kernel takes (p.Ap: more with one or four tiles)
+        const int regs = mt == 1 ? (nt == 1 ? (dot ? 72 : 64) : dot ? 96 : 72)
+                         : mt == 2 ? 96 : mt == 3 || (mt == 4 && !dot) ? 128 : 168;
+        const int resident = (int)std::min<size_t>(65536 / (regs * 32 * kMmaWarps), 227 * 1024 / (p.smem(Np) + 1024));
+        const double n = 0.4 * ((blocks + sms - 1) / sms) + 0.6 * std::max(per_sm, 1.0);
         const double gathers = p.eb() * ((Np + 3) / 4 * 4) / (6.0 * 32 * kMmaWarps);
-        const int resident = (int)std::min<size_t>(65536 / (regs[mt - 1] * 32 * kMmaWarps),
-                                                   227 * 1024 / (p.smem(Np) + 1024));
-        const double alone = steps * (mt * nt + 0.9 * mt + 3.6 * nt + 8) + 40 * std::ceil(gathers);
-        const double pipes = steps * (mt * nt + 0.2 * mt + 0.05) + 4 * gathers;
-        const double c = alone + (n - 1) * std::max(alone / resident, pipes);
-        if (c < cost) {
-          cost = c;
-          best = p;
+        const double steps = rounds * steps1;
+        const double alone = steps * (0.8 * mt * nt + mt + 3.6 * nt + 8) + 80 * std::ceil(gathers);
+        const double pipes = steps * (mt * nt + 0.2 * mt + 0.08) + 4 * gathers;
+        const double f = alone + (n - 1) * std::max(alone / resident, pipes);
+        if (r < rough_cost) {
+          rough_cost = r;
+          rough_fine = f;
+          rough = p;
+        }
+        if (f < fine_cost) {
+          fine_cost = f;
+          fine = p;
         }
       }
-  return best;
+  return fine_cost < (rough.gy > 1 ? 1.0 : 0.92) * rough_fine ? fine : rough;
 }
 
 template <int C, int MT, int NT>
@@ -442,7 +460,7 @@ static int launch_ax_simplex_mma(int N, int32_t E, const int32_t* elementList, c
                                  const double* q, double* Aq, const int* skip, cudaStream_t s, double* partials,
                                  int* nblocks) {
   const int Np = simplex_np(C == 4 ? 2 : 3, N);
-  const SimplexMmaPlan p = simplex_mma_plan(C, Np, E, sm_count());
+  const SimplexMmaPlan p = simplex_mma_plan(C, Np, E, sm_count(), partials != nullptr);
 #define BP_SIMPLEX_MMA(MT, NT)                                                                                     \
   if (p.mt == MT && p.nt == NT)                                                                                    \
     return launch_simplex_mma<C, MT, NT>(p, Np, E, elementList, G2L, wJ, ggeo, S, MM, lambda, q, Aq, skip, s, partials, \
@@ -497,7 +515,7 @@ static int launch_ax_simplex_any(int dim, int N, int32_t Nelements, const int32_
 void simplex_plan(int dim, int N, int32_t Nelements, int32_t* plan) {
   const int Np = simplex_np(dim, N);
   const SimplexMmaPlan p =
-      Np < 8 ? SimplexMmaPlan{0, 0, 0, 0} : simplex_mma_plan(dim == 2 ? 4 : 7, Np, Nelements, sm_count());
+      Np < 8 ? SimplexMmaPlan{0, 0, 0, 0} : simplex_mma_plan(dim == 2 ? 4 : 7, Np, Nelements, sm_count(), false);
   plan[0] = p.mt;
   plan[1] = p.nt;
   plan[2] = p.wm;

@@ -117,12 +117,12 @@ def _simplex_reference(gm, q):
 # (dim, degree, cells per direction) and the 8-node tiles, 8-element tiles and warps
 # along the nodes of the plan on 148 SMs.  The permuted list leaves elements out,
 # and the last tile partly empty in the one list or the other.
-PLANS = [(2, 3, 1, 1, 1, 1), (2, 6, 1, 1, 1, 2), (2, 9, 1, 1, 1, 4), (2, 4, 110, 1, 2, 2), (2, 6, 90, 1, 2, 4),
-         (2, 3, 44, 2, 1, 1), (2, 6, 33, 2, 1, 2), (2, 13, 17, 2, 1, 4), (2, 3, 90, 2, 2, 1), (2, 6, 110, 2, 2, 2),
-         (2, 9, 70, 2, 2, 4), (2, 5, 40, 3, 1, 1), (2, 7, 31, 3, 1, 2), (2, 10, 23, 3, 1, 4), (2, 10, 49, 3, 2, 1),
-         (2, 15, 35, 3, 2, 2), (3, 8, 7, 3, 2, 4), (2, 15, 29, 4, 1, 1), (3, 5, 9, 4, 1, 2), (2, 13, 30, 4, 1, 4),
-         (3, 8, 8, 4, 2, 2), (3, 9, 7, 4, 2, 4), (2, 13, 28, 5, 1, 1), (2, 11, 34, 5, 1, 2), (2, 15, 31, 5, 1, 4),
-         (3, 4, 14, 5, 2, 1), (2, 10, 60, 5, 2, 2), (2, 15, 43, 5, 2, 4)]
+PLANS = [(2, 3, 1, 1, 1, 1), (2, 6, 1, 1, 1, 2), (2, 9, 1, 1, 1, 4), (3, 2, 12, 1, 2, 2), (2, 6, 50, 1, 2, 4),
+         (2, 3, 43, 2, 1, 1), (2, 6, 33, 2, 1, 2), (2, 13, 17, 2, 1, 4), (2, 3, 110, 2, 2, 1), (2, 6, 80, 2, 2, 2),
+         (2, 9, 51, 2, 2, 4), (2, 5, 45, 3, 1, 1), (2, 7, 29, 3, 1, 2), (2, 10, 22, 3, 1, 4), (3, 3, 16, 3, 2, 1),
+         (2, 8, 80, 3, 2, 2), (3, 8, 7, 3, 2, 4), (2, 13, 26, 4, 1, 4), (2, 6, 120, 4, 2, 1), (3, 8, 8, 4, 2, 2),
+         (3, 9, 7, 4, 2, 4), (2, 7, 80, 5, 1, 1), (3, 9, 6, 5, 1, 2), (2, 15, 24, 5, 1, 4), (3, 4, 16, 5, 2, 1),
+         (2, 10, 80, 5, 2, 2), (3, 10, 7, 5, 2, 4)]
 
 
 def _simplex_mesh(gpu, dim, N, n):
