@@ -248,16 +248,19 @@ cg_alpha_kernel(int nparts, const double* __restrict__ parts, CgScalars* sc, dou
 //
 // Up to this many block partials every block of the gather-update adds them
 // for itself (the same order in each, so the same alpha) and the alpha kernel is
-// left out: a read of at most 8 KB from L2 against a launch with its own grid
+// left out: a read of at most 12 KB from L2 against a launch with its own grid
 // reduction.  The rule counts blocks of the operator, not rows.  Measured in one
 // process, p = 1..15, 1e4 to 3e6 rows, time per iteration of three kernels by
-// four: FP64 0.69-0.98; FP32 0.63-1.00 up to a million rows, 1.04 at 1000
-// elements of p=15 (3.3 million rows).  Above 1024 partials: FP64 0.92-0.98 up to
-// 1e5-3e5 rows, then even (p=1 1.18); FP32 loses 2-10% from 1e6 rows on.
+// four, up to 1024 partials: FP64 0.69-0.98; FP32 0.63-1.00 up to a million rows,
+// 1.04 at 1000 elements of p=15 (3.3 million rows).  1024 to 1800: FP64 0.91-0.99
+// (BP1 p=2, 12,167 elements, 1,521 partials: 19.8 us an iteration against 21.7);
+// FP32 0.99-1.06.  Beyond: FP64 0.90-0.98 up to 1e5-3e5 rows, then even (p=1 1.18);
+// FP32 loses 2-10% from 1e6 rows on.
 // Launched programmatically the folded gather gains up to a third of the
 // iteration up to 1e5 rows and changes nothing beyond.  Four packed lanes, four
 // sums in each block, lose (p=4 10^3 to 1e-8 6.43 -> 6.69 ms) and keep the kernel.
-constexpr int kFoldParts = 1024;
+template <class V>
+constexpr int kFoldParts = sizeof(V) == 8 ? 1536 : 1024;
 
 // p.Ap from the operator's block partials, the same bits in every thread of
 // every block (each block adds all of them in the same order).
@@ -851,7 +854,7 @@ static int enqueue_iteration(bp_solver_s* S, V* x, V* r, V* p, V* p_alt, V* AqL,
     fuse.partials = S->fuse_partials.ptr;
     BP_TRY(elem_apply<V>(S, o, p, AqL, &S->scal->done, s, &fuse, &nparts));
   }
-  const bool fold = nparts <= kFoldParts;
+  const bool fold = nparts <= kFoldParts<V>;
   if (!fold)
     BP_CUDA_TRY(launch_pdl(cg_alpha_kernel<1>, alpha_grid(nparts), kThreads, 0, s, nparts, S->fuse_partials.ptr,
                            S->scal, hist_alpha, S->partials.ptr, S->counter.ptr));
